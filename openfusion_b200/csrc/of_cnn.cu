@@ -52,7 +52,8 @@ constexpr long kActIn = 2L * kInH * kInW;
 constexpr long kAct[4] = {16L * 30 * 40, 32L * 15 * 20, 64L * 8 * 10, 128L * 4 * 5};
 
 // Workspace (per batch b): BF16 activations a1..a4, f1; FP32 output; FP32
-// gradients g1..g4, gf1, gout (activation-sized).
+// gradients g1..g4, gf1 (masked by their ReLU, rounded to TF32), gout; the
+// packed weights; the weight gradients' partial sums.
 struct CnnWs {
   bf16 *a[4];
   bf16 *f1;
@@ -60,15 +61,19 @@ struct CnnWs {
   float *g[4];
   float *gf1;
   float *gout;
-  float *loss;  // [b] per-sample losses, then their sum at [b]
-  float *part;  // split-K partial tiles of the tensor-core GEMMs
+  float *loss;  // [b] per-sample losses, then their mean at [b]
+  uint4 *fw;    // forward weight fragments
+  uint2 *bw;    // input-gradient weight fragments
+  float *part;  // partial sums of the weight gradients
   size_t total;
 };
-size_t mma_part_floats(int b);
+size_t train_frag_bytes(bool fwd);
+size_t train_part_floats(int b);
 inline size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 CnnWs ws_layout(void *base, int b) {
   CnnWs w;
-  char *p = (char *)base;
+  // (room to align the caller's pointer, which need not be)
+  char *p = (char *)a256((size_t)base);
   size_t off = 0;
   auto take = [&](size_t bytes) { char *q = p ? p + off : nullptr; off += a256(bytes); return q; };
   for (int l = 0; l < 4; ++l) w.a[l] = (bf16 *)take((size_t)b * kAct[l] * sizeof(bf16));
@@ -78,8 +83,10 @@ CnnWs ws_layout(void *base, int b) {
   w.gf1 = (float *)take((size_t)b * kF1Out * sizeof(float));
   w.gout = (float *)take((size_t)b * kF2Out * sizeof(float));
   w.loss = (float *)take((size_t)(b + 1) * sizeof(float));
-  w.part = (float *)take(mma_part_floats(b) * sizeof(float));
-  w.total = off;
+  w.fw = (uint4 *)take(train_frag_bytes(true));
+  w.bw = (uint2 *)take(train_frag_bytes(false));
+  w.part = (float *)take(train_part_floats(b) * sizeof(float));
+  w.total = off + 256;
   return w;
 }
 
@@ -201,326 +208,7 @@ __global__ void __launch_bounds__(256) k_fc_fwd(const bf16 *__restrict__ in,
   }
 }
 
-// ------------------------------------------------- tensor-core GEMMs --
-//
-// The training contractions as implicit GEMMs on the tensor cores:
-// D[m, n] = sum_k A(m, k) B(k, n) with A and B read through a problem
-// functor that gathers them from the layer's tensors (im2col on the fly, the
-// padding and the ReLU masks included). One warp computes a 16 x 32 tile of
-// D, four mma n8 subtiles sharing each A fragment, over a K range:
-//   - forward (BF16 weights and activations): mma.sync m16n8k16 BF16 x BF16
-//     with FP32 accumulation, the products the scalar kernels form, summed in
-//     another fixed order;
-//   - backward (FP32 gradients): mma.sync m16n8k8 TF32 x TF32 with FP32
-//     accumulation; BF16 operands are exact in TF32, an FP32 gradient is
-//     rounded to TF32 (cvt.rna, relative error below 2^-11).
-// Large reductions (the weight gradients sum over batch x pixels) are split
-// along K over blockIdx.y; each slice writes its partial tile and a second
-// kernel sums the slices in index order, so every result is reproducible bit
-// for bit. Fragment layouts (PTX ISA, mma.m16n8k16 / m16n8k8, g = lane / 4,
-// t = lane % 4): A row-major, B column-major, accumulators c0..c3 at
-// (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1).
-
-constexpr int kMmaWarps = 4;      // warps per CTA, one 16 x 32 tile each
-constexpr int kMmaNt = 4;         // n8 subtiles per warp tile
-constexpr int kMmaTileN = 8 * kMmaNt;
-constexpr long kMmaSliceK = 2048; // K per split slice of a long reduction
-constexpr int kMmaMaxSlices = 256;
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t *>(&v);
-}
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ void mma_bf16(float *c, const uint32_t *a, const uint32_t *b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-__device__ __forceinline__ void mma_tf32(float *c, const uint32_t *a, const uint32_t *b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// Warp tile (m0, n0) over k in [k0, k1): BF16 (KS = 16) or TF32 (KS = 8).
-// Elements outside [0, M) x [0, Kd) or [0, Kd) x [0, N) read as 0 (Kd: the
-// reduction length of the problem).
-template <class P, bool BF16>
-__device__ __forceinline__ void mma_tile(const P &p, int m0, int n0, long k0, long k1,
-                                         float (&c)[kMmaNt][4]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  constexpr int KS = BF16 ? 16 : 8;
-  const int ma = m0 + g, mb = m0 + g + 8;
-  for (long k = k0; k < k1; k += KS) {
-    uint32_t a[4];
-    if (BF16) {
-      const long ka = k + 2 * t, kb = k + 2 * t + 8;
-      a[0] = pack_bf16x2(p.a(ma, ka), p.a(ma, ka + 1));
-      a[1] = pack_bf16x2(p.a(mb, ka), p.a(mb, ka + 1));
-      a[2] = pack_bf16x2(p.a(ma, kb), p.a(ma, kb + 1));
-      a[3] = pack_bf16x2(p.a(mb, kb), p.a(mb, kb + 1));
-    } else {
-      a[0] = to_tf32(p.a(ma, k + t));
-      a[1] = to_tf32(p.a(mb, k + t));
-      a[2] = to_tf32(p.a(ma, k + t + 4));
-      a[3] = to_tf32(p.a(mb, k + t + 4));
-    }
-#pragma unroll
-    for (int j = 0; j < kMmaNt; ++j) {
-      const int n = n0 + 8 * j + g;
-      uint32_t b[2];
-      if (BF16) {
-        b[0] = pack_bf16x2(p.b(k + 2 * t, n), p.b(k + 2 * t + 1, n));
-        b[1] = pack_bf16x2(p.b(k + 2 * t + 8, n), p.b(k + 2 * t + 9, n));
-        mma_bf16(c[j], a, b);
-      } else {
-        b[0] = to_tf32(p.b(k + t, n));
-        b[1] = to_tf32(p.b(k + t + 4, n));
-        mma_tf32(c[j], a, b);
-      }
-    }
-  }
-}
-
-// Grid: x over the warp tiles (kMmaWarps per CTA), y over the K slices.
-// With one slice the tile goes through p.store(m, n, value); with several,
-// slice s writes part[(s * M + m) * N + n] and k_mma_reduce sums them.
-template <class P, bool BF16>
-__global__ void __launch_bounds__(32 * kMmaWarps) k_mma(P p, float *__restrict__ part) {
-  const int tiles_n = (p.N + kMmaTileN - 1) / kMmaTileN;
-  const int tiles = ((p.M + 15) / 16) * tiles_n;
-  const int tile = blockIdx.x * kMmaWarps + (threadIdx.x >> 5);
-  if (tile >= tiles) return;  // warp-uniform
-  const int m0 = (tile / tiles_n) * 16, n0 = (tile % tiles_n) * kMmaTileN;
-  const long slice = (p.Kd + gridDim.y - 1) / gridDim.y;
-  const long KS = BF16 ? 16 : 8;
-  const long k0 = ((long)blockIdx.y * slice) / KS * KS;
-  const long k1 = blockIdx.y + 1 == gridDim.y ? p.Kd : (((long)blockIdx.y + 1) * slice) / KS * KS;
-  float c[kMmaNt][4] = {};
-  mma_tile<P, BF16>(p, m0, n0, k0, k1, c);
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int j = 0; j < kMmaNt; ++j)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int m = m0 + g + (r >= 2 ? 8 : 0), n = n0 + 8 * j + 2 * t + (r & 1);
-      if (m >= p.M || n >= p.N) continue;
-      if (gridDim.y == 1) p.store(m, n, c[j][r]);
-      else part[((size_t)blockIdx.y * p.M + m) * p.N + n] = c[j][r];
-    }
-}
-
-template <class P>
-__global__ void __launch_bounds__(256) k_mma_reduce(P p, const float *__restrict__ part,
-                                                    int slices) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)p.M * p.N) return;
-  float acc = 0.f;
-  for (int s = 0; s < slices; ++s) acc += part[(size_t)s * p.M * p.N + i];
-  p.store((int)(i / p.N), (int)(i % p.N), acc);
-}
-
-// K slices of a reduction of length K (1 when it is short).
-inline int mma_slices(long K) {
-  const long s = (K + kMmaSliceK - 1) / kMmaSliceK;
-  return (int)(s < 1 ? 1 : (s > kMmaMaxSlices ? kMmaMaxSlices : s));
-}
-
-// Launches D = A B of problem p; `part` holds slices x M x N floats when the
-// reduction is split.
-template <class P, bool BF16>
-void mma_launch(const P &p, float *part, int slices, cudaStream_t s) {
-  const long tiles = (long)((p.M + 15) / 16) * ((p.N + kMmaTileN - 1) / kMmaTileN);
-  dim3 grid((unsigned)((tiles + kMmaWarps - 1) / kMmaWarps), (unsigned)slices);
-  k_mma<P, BF16><<<grid, 32 * kMmaWarps, 0, s>>>(p, part);
-  if (slices > 1)
-    k_mma_reduce<P><<<(unsigned)(((long)p.M * p.N + 255) / 256), 256, 0, s>>>(p, part, slices);
-}
-
-// Convolution forward: m = co, k = (ci, ky, kx), n = (b, oy, ox);
-// out = relu(bias + acc) in BF16.
-template <int K, int S, int P>
-struct ConvFwdProb {
-  const bf16 *in, *wt;
-  const float *bias;
-  bf16 *out;
-  ConvSpec c;
-  int M, N;
-  long Kd;
-  __device__ float a(int m, long k) const {
-    return (m < M && k < Kd) ? bf(wt[(size_t)m * Kd + k]) : 0.f;
-  }
-  __device__ float b(long k, int n) const {
-    if (n >= N || k >= Kd) return 0.f;
-    const int ci = (int)(k / (K * K)), ky = (int)((k / K) % K), kx = (int)(k % K);
-    const int hw = c.ho * c.wo, bb = n / hw, p = n % hw, oy = p / c.wo, ox = p % c.wo;
-    const int iy = oy * S - P + ky, ix = ox * S - P + kx;
-    if ((unsigned)iy >= (unsigned)c.hi || (unsigned)ix >= (unsigned)c.wi) return 0.f;
-    return bf(in[(((size_t)bb * c.ci + ci) * c.hi + iy) * c.wi + ix]);
-  }
-  __device__ void store(int m, int n, float v) const {
-    const int hw = c.ho * c.wo, bb = n / hw, p = n % hw;
-    out[((size_t)bb * c.co + m) * hw + p] = __float2bfloat16_rn(fmaxf(v + bias[m], 0.f));
-  }
-};
-
-// The gradient at a ReLU layer's pre-activation: gpost where act > 0.
-__device__ __forceinline__ float relu_grad(const float *gpost, const bf16 *act, size_t o) {
-  return (!act || bf(act[o]) > 0.f) ? gpost[o] : 0.f;
-}
-
-// Convolution input gradient: m = ci, k = (co, ky, kx), n = (b, iy, ix).
-template <int K, int S, int P>
-struct ConvBwdDataProb {
-  const float *gpost;
-  const bf16 *act, *wt;
-  float *gin;
-  ConvSpec c;
-  int M, N;
-  long Kd;
-  __device__ float a(int m, long k) const {
-    if (m >= M || k >= Kd) return 0.f;
-    const int co = (int)(k / (K * K)), tap = (int)(k % (K * K));
-    return bf(wt[((size_t)co * c.ci + m) * K * K + tap]);
-  }
-  __device__ float b(long k, int n) const {
-    if (n >= N || k >= Kd) return 0.f;
-    const int co = (int)(k / (K * K)), ky = (int)((k / K) % K), kx = (int)(k % K);
-    const int hw = c.hi * c.wi, bb = n / hw, q = n % hw, iy = q / c.wi, ix = q % c.wi;
-    const int ny = iy + P - ky, nx = ix + P - kx;
-    if (ny < 0 || nx < 0 || ny % S || nx % S) return 0.f;
-    const int oy = ny / S, ox = nx / S;
-    if (oy >= c.ho || ox >= c.wo) return 0.f;
-    return relu_grad(gpost, act, (((size_t)bb * c.co + co) * c.ho + oy) * c.wo + ox);
-  }
-  __device__ void store(int m, int n, float v) const {
-    const int hw = c.hi * c.wi, bb = n / hw, q = n % hw;
-    gin[((size_t)bb * c.ci + m) * hw + q] = v;
-  }
-};
-
-// Convolution weight (and bias) gradient: m = co, k = (b, oy, ox),
-// n = (ci, ky, kx), and n = ci K K is the bias (B = 1).
-template <int K, int S, int P>
-struct ConvBwdWeightProb {
-  const float *gpost;
-  const bf16 *act, *in;
-  float *gw, *gbias;
-  ConvSpec c;
-  int M, N;
-  long Kd;
-  __device__ float a(int m, long k) const {
-    if (m >= M || k >= Kd) return 0.f;
-    const int hw = c.ho * c.wo, bb = (int)(k / hw), p = (int)(k % hw);
-    return relu_grad(gpost, act, ((size_t)bb * c.co + m) * hw + p);
-  }
-  __device__ float b(long k, int n) const {
-    if (n >= N || k >= Kd) return 0.f;
-    if (n == N - 1) return 1.f;
-    const int ci = n / (K * K), ky = (n / K) % K, kx = n % K;
-    const int hw = c.ho * c.wo, bb = (int)(k / hw), p = (int)(k % hw), oy = p / c.wo, ox = p % c.wo;
-    const int iy = oy * S - P + ky, ix = ox * S - P + kx;
-    if ((unsigned)iy >= (unsigned)c.hi || (unsigned)ix >= (unsigned)c.wi) return 0.f;
-    return bf(in[(((size_t)bb * c.ci + ci) * c.hi + iy) * c.wi + ix]);
-  }
-  __device__ void store(int m, int n, float v) const {
-    if (n == N - 1) gbias[m] = v;
-    else gw[(size_t)m * (N - 1) + n] = v;
-  }
-};
-
-// Fully connected forward: m = j, k = i, n = b; out = act(bias + acc).
-template <bool RELU, typename TOut>
-struct FcFwdProb {
-  const bf16 *in, *wt;
-  const float *bias;
-  TOut *out;
-  int M, N;
-  long Kd;
-  __device__ float a(int m, long k) const {
-    return (m < M && k < Kd) ? bf(wt[(size_t)m * Kd + k]) : 0.f;
-  }
-  __device__ float b(long k, int n) const {
-    return (n < N && k < Kd) ? bf(in[(size_t)n * Kd + k]) : 0.f;
-  }
-  __device__ void store(int m, int n, float v) const {
-    v += bias[m];
-    if (RELU) v = fmaxf(v, 0.f);
-    if constexpr (sizeof(TOut) == 2) out[(size_t)n * M + m] = __float2bfloat16_rn(v);
-    else out[(size_t)n * M + m] = v;
-  }
-};
-
-// Fully connected input gradient: m = i, k = j, n = b.
-struct FcBwdDataProb {
-  const float *gpost;
-  const bf16 *act, *wt;
-  float *gin;
-  int M, N;  // M = nin, N = batch
-  long Kd;   // nout
-  __device__ float a(int m, long k) const {
-    return (m < M && k < Kd) ? bf(wt[(size_t)k * M + m]) : 0.f;
-  }
-  __device__ float b(long k, int n) const {
-    return (n < N && k < Kd) ? relu_grad(gpost, act, (size_t)n * Kd + k) : 0.f;
-  }
-  __device__ void store(int m, int n, float v) const { gin[(size_t)n * M + m] = v; }
-};
-
-// Fully connected weight (and bias) gradient: m = j, k = b, n = i, and
-// n = nin is the bias (B = 1).
-struct FcBwdWeightProb {
-  const float *gpost;
-  const bf16 *act, *in;
-  float *gw, *gbias;
-  int M, N;  // M = nout, N = nin + 1
-  long Kd;   // batch
-  __device__ float a(int m, long k) const {
-    return (m < M && k < Kd) ? relu_grad(gpost, act, (size_t)k * M + m) : 0.f;
-  }
-  __device__ float b(long k, int n) const {
-    if (n >= N || k >= Kd) return 0.f;
-    return n == N - 1 ? 1.f : bf(in[(size_t)k * (N - 1) + n]);
-  }
-  __device__ void store(int m, int n, float v) const {
-    if (n == N - 1) gbias[m] = v;
-    else gw[(size_t)m * (N - 1) + n] = v;
-  }
-};
-
-// ----------------------------------------------------------------- loss --
-
-// Mean over the batch of sum_k wk (out - target)^2; gout = d loss / d out.
-// loss[b] per sample, loss[batch] the mean (fixed-order sum, one thread).
-__global__ void k_loss(const float *__restrict__ out, const float *__restrict__ target,
-                       const float *__restrict__ wk, int batch, float *__restrict__ gout,
-                       float *__restrict__ loss) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < batch) {
-    float l = 0.f;
-    for (int k = 0; k < kF2Out; ++k) {
-      const float e = out[b * kF2Out + k] - target[b * kF2Out + k];
-      l = fmaf(wk[k] * e, e, l);
-      gout[b * kF2Out + k] = 2.f * wk[k] * e / (float)batch;
-    }
-    loss[b] = l;
-  }
-}
-__global__ void k_loss_sum(float *loss, int batch) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  float s = 0.f;
-  for (int b = 0; b < batch; ++b) s += loss[b];
-  loss[batch] = s / (float)batch;
-}
+#include "of_cnn_train.cuh"
 
 // ---------------------------------------------------------- init / adam --
 
@@ -567,84 +255,76 @@ __global__ void k_adam(float *__restrict__ master, bf16 *__restrict__ mirror,
   mirror[i] = __float2bfloat16_rn(p);
 }
 
-unsigned blocks_for(long n) { return (unsigned)((n + 255) / 256 < 148L * 64 ? (n + 255) / 256 : 148L * 64); }
-
 constexpr int kSmallBatch = 16;  // up to this batch, one warp per conv / fc output
 
-// Partial-tile floats the split reductions of a batch need (the weight
-// gradients, whose K = batch x output pixels).
-size_t mma_part_floats(int b) {
-  size_t m = 0;
-  for (int l = 0; l < 4; ++l) {
-    const ConvSpec &c = kConv[l];
-    const int sl = mma_slices((long)b * c.ho * c.wo);
-    const int taps = (l == 0 ? 25 : 9) * c.ci;
-    if (sl > 1) m = m > (size_t)sl * c.co * (taps + 1) ? m : (size_t)sl * c.co * (taps + 1);
-  }
-  const int sl = mma_slices(b);
-  if (sl > 1) {
-    const size_t f1 = (size_t)sl * kF1Out * (kF1In + 1), f2 = (size_t)sl * kF2Out * (kF1Out + 1);
-    m = m > f1 ? m : f1;
-    m = m > f2 ? m : f2;
-  }
-  return m;
+size_t train_frag_bytes(bool fwd) {
+  return fwd ? (size_t)kFwFrags * 32 * sizeof(uint4) : (size_t)kBwFrags * 32 * sizeof(uint2);
 }
+size_t train_part_floats(int b) { return (size_t)wg_plan(b).total; }
 
 template <int K, int S, int P>
-void conv_fwd(const bf16 *in, const bf16 *w, const float *b, const ConvSpec &c, int batch, bf16 *out,
-              float *part, cudaStream_t s) {
+void conv_fwd_small(const bf16 *in, const bf16 *w, const float *b, const ConvSpec &c, int batch,
+                    bf16 *out, cudaStream_t s) {
   const long n = (long)batch * c.co * c.ho * c.wo;
-  if (batch <= kSmallBatch) {
-    k_conv_fwd_warp<K, S, P><<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(in, w, b, c, batch, out);
-  } else {
-    ConvFwdProb<K, S, P> p{in, w, b, out, c, c.co, batch * c.ho * c.wo, (long)c.ci * K * K};
-    mma_launch<ConvFwdProb<K, S, P>, true>(p, part, 1, s);
-  }
+  k_conv_fwd_warp<K, S, P><<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(in, w, b, c, batch, out);
 }
 
-void forward(const bf16 *pw, const float *pm, const bf16 *in, int batch, const CnnWs &w,
-             cudaStream_t s) {
-  const bf16 *x = in;
-  conv_fwd<5, 2, 2>(x, pw + kOffW0, pm + kOffB0, kConv[0], batch, w.a[0], w.part, s);
-  conv_fwd<3, 2, 1>(w.a[0], pw + kOffW1, pm + kOffB1, kConv[1], batch, w.a[1], w.part, s);
-  conv_fwd<3, 2, 1>(w.a[1], pw + kOffW2, pm + kOffB2, kConv[2], batch, w.a[2], w.part, s);
-  conv_fwd<3, 2, 1>(w.a[2], pw + kOffW3, pm + kOffB3, kConv[3], batch, w.a[3], w.part, s);
-  if (batch <= kSmallBatch) {
+// The dynamic shared memory of a training kernel (set on every call: the
+// attribute belongs to the current context).
+template <typename Kernel>
+cudaError_t opt_in(Kernel *k, size_t bytes) {
+  return cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+// Images a block of the conv chains takes at a time: 2 once a wave of
+// single-image blocks (one an SM) would not hold the batch. At 148 images and
+// below one image a block keeps every block in the first wave; above, two
+// images share each weight fragment and fill conv4's 8-pixel tiles.
+inline int chain_images(int batch) { return batch > of::kSmCount ? 2 : 1; }
+
+// One launch of a conv chain kernel over the batch: its blocks loop over
+// images when the batch exceeds one wave.
+template <int NI, typename... P, typename... A>
+cudaError_t launch_chain(void (*k)(P...), size_t smem, int batch, cudaStream_t s, A... args) {
+  cudaError_t e = opt_in(k, smem);
+  if (e != cudaSuccess) return e;
+  const int want = (batch + NI - 1) / NI;
+  k<<<want < of::kSmCount ? want : of::kSmCount, kTrThreads, smem, s>>>(args...);
+  return cudaSuccess;
+}
+
+// Forward pass; with `target` also the loss and the gradient at FC1's output
+// (the head kernel computes both), and the input-gradient weight fragments.
+cudaError_t forward(const bf16 *pw, const float *pm, const bf16 *in, int batch, const CnnWs &w,
+                    cudaStream_t s, const float *target, const float *wk) {
+  const bool small = batch <= kSmallBatch;
+  cudaError_t e = cudaSuccess;
+  const int frags = kFwFrags + (target ? kBwFrags : 0);
+  if (!small || target)
+    k_cnn_pack<<<(frags * 32 + 255) / 256, 256, 0, s>>>(pw, w.fw, target ? w.bw : nullptr);
+  if (small) {
+    conv_fwd_small<5, 2, 2>(in, pw + kOffW0, pm + kOffB0, kConv[0], batch, w.a[0], s);
+    conv_fwd_small<3, 2, 1>(w.a[0], pw + kOffW1, pm + kOffB1, kConv[1], batch, w.a[1], s);
+    conv_fwd_small<3, 2, 1>(w.a[1], pw + kOffW2, pm + kOffB2, kConv[2], batch, w.a[2], s);
+    conv_fwd_small<3, 2, 1>(w.a[2], pw + kOffW3, pm + kOffB3, kConv[3], batch, w.a[3], s);
     const long w1 = (long)batch * kF1Out * 32, w2 = (long)batch * kF2Out * 32;
     k_fc_fwd<true, bf16><<<(unsigned)((w1 + 255) / 256), 256, 0, s>>>(
         w.a[3], pw + kOffF1, pm + kOffBF1, kF1In, kF1Out, batch, w.f1);
     k_fc_fwd<false, float><<<(unsigned)((w2 + 255) / 256), 256, 0, s>>>(
         w.f1, pw + kOffF2, pm + kOffBF2, kF1Out, kF2Out, batch, w.out);
   } else {
-    FcFwdProb<true, bf16> f1{w.a[3], pw + kOffF1, pm + kOffBF1, w.f1, kF1Out, batch, kF1In};
-    mma_launch<FcFwdProb<true, bf16>, true>(f1, w.part, 1, s);
-    FcFwdProb<false, float> f2{w.f1, pw + kOffF2, pm + kOffBF2, w.out, kF2Out, batch, kF1Out};
-    mma_launch<FcFwdProb<false, float>, true>(f2, w.part, 1, s);
+    const bool words = ((uintptr_t)in & 3u) == 0;
+    e = chain_images(batch) == 2
+            ? launch_chain<2>(k_conv_fwd<2>, sizeof(FwdSmem<2>), batch, s, in, (const uint4 *)w.fw,
+                              pm, batch, words, w.a[0], w.a[1], w.a[2], w.a[3])
+            : launch_chain<1>(k_conv_fwd<1>, sizeof(FwdSmem<1>), batch, s, in, (const uint4 *)w.fw,
+                              pm, batch, words, w.a[0], w.a[1], w.a[2], w.a[3]);
+    if (e != cudaSuccess) return e;
   }
-}
-
-// A convolution's weight and bias gradients and, when gin is given, its
-// input gradient, from the gradient at its output (masked by its ReLU).
-template <int K, int S, int P>
-void conv_bwd(const float *gpost, const bf16 *act, const bf16 *in, const bf16 *wt, const ConvSpec &c,
-              int batch, float *gin, float *gw, float *gb, float *part, cudaStream_t s) {
-  ConvBwdWeightProb<K, S, P> pw{gpost, act, in, gw, gb, c, c.co, c.ci * K * K + 1,
-                                (long)batch * c.ho * c.wo};
-  mma_launch<ConvBwdWeightProb<K, S, P>, false>(pw, part, mma_slices(pw.Kd), s);
-  if (gin) {
-    ConvBwdDataProb<K, S, P> pd{gpost, act, wt, gin, c, c.ci, batch * c.hi * c.wi,
-                                (long)c.co * K * K};
-    mma_launch<ConvBwdDataProb<K, S, P>, false>(pd, part, 1, s);
-  }
-}
-
-// A fully connected layer's weight and bias gradients and its input gradient.
-void fc_bwd(const float *gpost, const bf16 *act, const bf16 *in, const bf16 *wt, int nin, int nout,
-            int batch, float *gin, float *gw, float *gb, float *part, cudaStream_t s) {
-  FcBwdWeightProb pw{gpost, act, in, gw, gb, nout, nin + 1, batch};
-  mma_launch<FcBwdWeightProb, false>(pw, part, mma_slices(batch), s);
-  FcBwdDataProb pd{gpost, act, wt, gin, nin, batch, nout};
-  mma_launch<FcBwdDataProb, false>(pd, part, 1, s);
+  if (!small || target)
+    k_head<<<(batch + kHeadN - 1) / kHeadN, kHeadThreads, 0, s>>>(
+        w.a[3], w.fw, pw, pm, batch, small, w.f1, w.out, target, wk, w.gout, w.gf1, w.loss);
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -688,7 +368,8 @@ extern "C" of_status_t of_cnn_forward(const uint16_t *d_params, const float *d_m
   if (!d_params || !d_master || !d_input || !d_ws || batch < 1 || batch > 65536)
     return OF_ERR_INVALID_ARGUMENT;
   CnnWs w = ws_layout(d_ws, batch);
-  forward((const bf16 *)d_params, d_master, (const bf16 *)d_input, batch, w, (cudaStream_t)s);
+  OF_CUDA_TRY(forward((const bf16 *)d_params, d_master, (const bf16 *)d_input, batch, w,
+                      (cudaStream_t)s, nullptr, nullptr));
   if (d_out)
     OF_CUDA_TRY(cudaMemcpyAsync(d_out, w.out, (size_t)batch * kF2Out * sizeof(float),
                                 cudaMemcpyDeviceToDevice, (cudaStream_t)s));
@@ -706,26 +387,29 @@ extern "C" of_status_t of_cnn_backward(const uint16_t *d_params, const float *d_
   const bf16 *pw = (const bf16 *)d_params;
   const bf16 *in = (const bf16 *)d_input;
   CnnWs w = ws_layout(d_ws, batch);
-  forward(pw, d_master, in, batch, w, s);
-  k_loss<<<(batch + 255) / 256, 256, 0, s>>>(w.out, d_target, d_loss_weights, batch, w.gout, w.loss);
-  k_loss_sum<<<1, 32, 0, s>>>(w.loss, batch);
-  // f2 (linear): gradients of its weights and of f1's output
-  fc_bwd(w.gout, nullptr, w.f1, pw + kOffF2, kF1Out, kF2Out, batch, w.gf1, d_grad + kOffF2,
-         d_grad + kOffBF2, w.part, s);
-  // f1 (ReLU)
-  fc_bwd(w.gf1, w.f1, w.a[3], pw + kOffF1, kF1In, kF1Out, batch, w.g[3], d_grad + kOffF1,
-         d_grad + kOffBF1, w.part, s);
-  // convs (ReLU), last to first; the first has no input gradient
-  conv_bwd<3, 2, 1>(w.g[3], w.a[3], w.a[2], pw + kOffW3, kConv[3], batch, w.g[2], d_grad + kOffW3,
-                    d_grad + kOffB3, w.part, s);
-  conv_bwd<3, 2, 1>(w.g[2], w.a[2], w.a[1], pw + kOffW2, kConv[2], batch, w.g[1], d_grad + kOffW2,
-                    d_grad + kOffB2, w.part, s);
-  conv_bwd<3, 2, 1>(w.g[1], w.a[1], w.a[0], pw + kOffW1, kConv[1], batch, w.g[0], d_grad + kOffW1,
-                    d_grad + kOffB1, w.part, s);
-  conv_bwd<5, 2, 2>(w.g[0], w.a[0], in, pw + kOffW0, kConv[0], batch, nullptr, d_grad + kOffW0,
-                    d_grad + kOffB0, w.part, s);
-  if (d_loss)
-    OF_CUDA_TRY(cudaMemcpyAsync(d_loss, w.loss + batch, sizeof(float), cudaMemcpyDeviceToDevice, s));
+  OF_CUDA_TRY(forward(pw, d_master, in, batch, w, s, d_target, d_loss_weights));
+  // FC1's input gradient, both FC layers' weight gradients
+  const int dgrad = ((batch + kFcPairs - 1) / kFcPairs) * (kF1In / 128);
+  k_fc_bwd<<<dgrad + kF1WBlocks + 1 + kFcBiasBlocks, kFcThreads, 0, s>>>(
+      w.gf1, w.gout, w.a[3], w.f1, pw, batch, dgrad, w.g[3], d_grad);
+  // conv4..conv2 input gradients (conv1 has none)
+  OF_CUDA_TRY(chain_images(batch) == 2
+                  ? launch_chain<2>(k_conv_dgrad<2>, sizeof(BwdSmem<2>), batch, s,
+                                    (const float *)w.g[3], (const uint2 *)w.bw, batch,
+                                    (const bf16 *)w.a[0], (const bf16 *)w.a[1], (const bf16 *)w.a[2],
+                                    w.g[0], w.g[1], w.g[2])
+                  : launch_chain<1>(k_conv_dgrad<1>, sizeof(BwdSmem<1>), batch, s,
+                                    (const float *)w.g[3], (const uint2 *)w.bw, batch,
+                                    (const bf16 *)w.a[0], (const bf16 *)w.a[1], (const bf16 *)w.a[2],
+                                    w.g[0], w.g[1], w.g[2]));
+  // conv weight gradients and the mean loss
+  const WgPlan plan = wg_plan(batch);
+  const WgArgs A = {{in, w.a[0], w.a[1], w.a[2]}, {w.g[0], w.g[1], w.g[2], w.g[3]}};
+  OF_CUDA_TRY(opt_in(k_conv_wgrad, kWgSmem));
+  k_conv_wgrad<<<plan.first[4], kTrThreads, kWgSmem, s>>>(A, plan, batch,
+                                                          ((uintptr_t)in & 3u) == 0, w.part);
+  k_wgrad_reduce<<<(unsigned)((kOffF1 + 255) / 256) + 1, 256, 0, s>>>(plan, w.part, d_grad, w.loss,
+                                                                      batch, d_loss);
   return of_launch_status();
 }
 

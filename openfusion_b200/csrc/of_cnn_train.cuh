@@ -1,0 +1,956 @@
+// of_cnn_train.cuh -- forward and backward of the warm-start CNN for batches
+// (training, and inference above kSmallBatch), included by of_cnn.cu after the
+// layer table, the parameter offsets and the workspace.
+//
+// Every contraction is an implicit GEMM D[m, n] = sum_k A(m, k) B(k, n) on
+// mma.sync tensor-core tiles: forward m16n8k16 BF16 x BF16, backward m16n8k8
+// TF32 x TF32 (BF16 operands are exact in TF32, an FP32 gradient is rounded
+// with cvt.rna, relative error below 2^-11), FP32 accumulation. The layers are
+// small (5.7 M multiply-adds a pair), so tensor throughput is never the bound;
+// what bounds a step is how the operands reach the fragments. Here a block
+// holds the images it works on in shared memory as zero-padded planes
+// [channel][image][row][column], so that an operand element sits at
+// (offset of its pixel) + (offset of its tap): two table look-ups and an add,
+// no division and no border test. The weights are packed once per call into
+// fragment order (one vector load a lane and k step). The legacy mma.sync form
+// is kept because its sums are: the forward pass and the input gradients round
+// to BF16 / TF32 between layers, so a different order of accumulation moves
+// single activations by one rounding step and the gradients by 1e-4.
+// Launches of a training step: pack, conv1..4, FC1 + FC2 + loss, FC backward,
+// conv4..2 input gradients, conv weight gradients, their reduction (7, and
+// Adam). Measured on B200 at batch 256 (time of the step, Adam included):
+// per-element gathers with divisions, one warp a tile, 8065 us; this form
+// 293 us.
+//
+// Fragment layouts (PTX ISA, mma.m16n8k16 / m16n8k8, g = lane / 4, t = lane %
+// 4): A row-major, B column-major, accumulators c0..c3 at (g, 2t), (g, 2t + 1),
+// (g + 8, 2t), (g + 8, 2t + 1).
+#pragma once
+
+constexpr int kTrThreads = 512;
+constexpr size_t kAct0 = kAct[0], kAct1 = kAct[1], kAct2 = kAct[2], kAct3 = kAct[3];
+constexpr int kTrWarps = kTrThreads / 32;
+
+__device__ __forceinline__ float to_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
+}
+__device__ __forceinline__ void mma_bf16(float *c, const uint4 &a, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_tf32(float *c, float a0, float a1, float a2, float a3, float b0,
+                                         float b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)),
+        "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+__device__ __forceinline__ float bits_f(uint32_t b16) { return __uint_as_float(b16 << 16); }
+
+// ------------------------------------------------------- packed weights --
+// Forward fragments: one uint4 a lane for each (m tile, k16 step): the words
+// (row g, k 2t..), (row g + 8, k 2t..), (row g, k 2t + 8..), (row g + 8, ..),
+// zero beyond K and M. Layers conv1..4, FC1, FC2.
+constexpr int fw_m(int l) { return l < 4 ? kConv[l].co : (l == 4 ? kF1Out : kF2Out); }
+constexpr int fw_k(int l) {
+  return l < 4 ? kConv[l].ci * kConv[l].k * kConv[l].k : (l == 4 ? kF1In : kF1Out);
+}
+constexpr int fw_mt(int l) { return (fw_m(l) + 15) / 16; }
+constexpr int fw_ks(int l) { return (fw_k(l) + 15) / 16; }
+constexpr int fw_first(int l) { return l == 0 ? 0 : fw_first(l - 1) + fw_mt(l - 1) * fw_ks(l - 1); }
+constexpr long fw_off(int l) {
+  return l == 0 ? kOffW0 : l == 1 ? kOffW1 : l == 2 ? kOffW2 : l == 3 ? kOffW3 : l == 4 ? kOffF1 : kOffF2;
+}
+constexpr int kFwFrags = fw_first(6);
+// Input-gradient fragments of conv2..4: one uint2 a lane for each (m tile, k8
+// step), m = ci, k = (co, tap): {(g, t) | (g + 8, t) << 16, (g, t + 4) |
+// (g + 8, t + 4) << 16}.
+constexpr int bw_mt(int l) { return kConv[l].ci / 16; }
+constexpr int bw_ks(int l) { return kConv[l].co * 9 / 8; }
+constexpr int bw_first(int l) { return l <= 1 ? 0 : bw_first(l - 1) + bw_mt(l - 1) * bw_ks(l - 1); }
+constexpr int kBwFrags = bw_first(4);
+static_assert(fw_ks(1) * 16 == fw_k(1) && fw_ks(2) * 16 == fw_k(2) && fw_ks(3) * 16 == fw_k(3) &&
+                  fw_ks(4) * 16 == fw_k(4) && fw_ks(5) * 16 == fw_k(5), "only conv1 pads K");
+
+template <int L>
+__device__ __forceinline__ uint4 fw_frag(const bf16 *pw, int f, int lane) {
+  const unsigned short *w = reinterpret_cast<const unsigned short *>(pw + fw_off(L));
+  const int mt = f / fw_ks(L), ks = f % fw_ks(L), g = lane >> 2, t = lane & 3;
+  auto word = [&](int m, int k) -> uint32_t {
+    uint32_t lo = 0, hi = 0;
+    if (m < fw_m(L) && k < fw_k(L)) lo = w[(size_t)m * fw_k(L) + k];
+    if (m < fw_m(L) && k + 1 < fw_k(L)) hi = w[(size_t)m * fw_k(L) + k + 1];
+    return lo | hi << 16;
+  };
+  const int m = mt * 16 + g, k = ks * 16 + 2 * t;
+  return make_uint4(word(m, k), word(m + 8, k), word(m, k + 8), word(m + 8, k + 8));
+}
+template <int L>
+__device__ __forceinline__ uint2 bw_frag(const bf16 *pw, int f, int lane) {
+  const unsigned short *w = reinterpret_cast<const unsigned short *>(pw + fw_off(L));
+  const int mt = f / bw_ks(L), ks = f % bw_ks(L), g = lane >> 2, t = lane & 3;
+  auto el = [&](int m, int k) -> uint32_t { return w[((k / 9) * kConv[L].ci + m) * 9 + k % 9]; };
+  const int m = mt * 16 + g, k = ks * 8 + t;
+  return make_uint2(el(m, k) | el(m + 8, k) << 16, el(m, k + 4) | el(m + 8, k + 4) << 16);
+}
+
+// One thread a fragment lane: 2-byte reads (a caller's parameter buffer needs
+// no wider alignment), coalesced vector stores.
+__global__ void __launch_bounds__(256) k_cnn_pack(const bf16 *__restrict__ pw,
+                                                  uint4 *__restrict__ fw, uint2 *__restrict__ bw) {
+  const int i = blockIdx.x * 256 + threadIdx.x, f = i >> 5, lane = i & 31;
+  if (f < kFwFrags) {
+    uint4 v;
+    if (f < fw_first(1)) v = fw_frag<0>(pw, f - fw_first(0), lane);
+    else if (f < fw_first(2)) v = fw_frag<1>(pw, f - fw_first(1), lane);
+    else if (f < fw_first(3)) v = fw_frag<2>(pw, f - fw_first(2), lane);
+    else if (f < fw_first(4)) v = fw_frag<3>(pw, f - fw_first(3), lane);
+    else if (f < fw_first(5)) v = fw_frag<4>(pw, f - fw_first(4), lane);
+    else v = fw_frag<5>(pw, f - fw_first(5), lane);
+    fw[i] = v;
+  } else if (bw && f < kFwFrags + kBwFrags) {
+    const int q = f - kFwFrags;
+    uint2 v;
+    if (q < bw_first(2)) v = bw_frag<1>(pw, q - bw_first(1), lane);
+    else if (q < bw_first(3)) v = bw_frag<2>(pw, q - bw_first(2), lane);
+    else v = bw_frag<3>(pw, q - bw_first(3), lane);
+    bw[q * 32 + lane] = v;
+  }
+}
+
+// ------------------------------------------------------- padded planes --
+// The input of conv layer L in shared memory: [channel][image][PH][PW], the
+// image at row P, column 2 (an even column, so that pixel pairs stay one
+// word), zeros around it. Tap (ky, kx) of output pixel (oy, ox) lies at
+// (oy S) PW + ox S + (2 - P) + ky PW + kx.
+constexpr int plane_h(int l) { return (kConv[l].ho - 1) * kConv[l].s + kConv[l].k; }
+constexpr int plane_w(int l) {
+  const int need = (kConv[l].wo - 1) * kConv[l].s + kConv[l].k + 2 - kConv[l].p;
+  return ((need > kConv[l].wi + 2 ? need : kConv[l].wi + 2) + 1) / 2 * 2;
+}
+constexpr int plane_n(int l) { return plane_h(l) * plane_w(l); }
+static_assert(plane_h(0) >= 62 && plane_h(1) >= 31 && plane_h(2) >= 16 && plane_h(3) >= 9,
+              "the planes hold every input row");
+
+// Offsets of a lane's four taps of a forward k16 step: k = 16 s + {2t, 2t + 1,
+// 2t + 8, 2t + 9}.
+template <int L, int NI>
+__device__ __forceinline__ int tap_offset(int k) {
+  constexpr int KK = kConv[L].k * kConv[L].k;
+  if (k >= fw_k(L)) return 0;  // (padding of K: its operand is zeroed)
+  const int ci = k / KK, ky = (k % KK) / kConv[L].k, kx = k % kConv[L].k;
+  return ci * NI * plane_n(L) + ky * plane_w(L) + kx;
+}
+template <int L, int NI>
+__device__ __forceinline__ void fill_taps(ushort4 *tab) {
+  static_assert(kConv[L].ci * NI * plane_n(L) < 65536, "16-bit offsets");
+  for (int i = threadIdx.x; i < fw_ks(L) * 4; i += kTrThreads) {
+    const int k = (i >> 2) * 16 + 2 * (i & 3);
+    tab[i] = make_ushort4(tap_offset<L, NI>(k), tap_offset<L, NI>(k + 1), tap_offset<L, NI>(k + 8),
+                          tap_offset<L, NI>(k + 9));
+  }
+}
+
+// `n` images of a BF16 NCHW tensor (all CT channels, those from c0 .. c0 + CC)
+// into planes; images beyond `n` are zeroed. Row pairs as words, or element
+// by element when the tensor is not word-aligned.
+template <int L, int NI, int CC, int THREADS>
+__device__ __forceinline__ void stage_images(const bf16 *__restrict__ src, int n, int c0,
+                                             bf16 *__restrict__ s, bool words) {
+  constexpr int H = kConv[L].hi, W = kConv[L].wi, CT = kConv[L].ci, P = kConv[L].p;
+  constexpr int WW = W / 2, T = CC * NI * H * WW;
+  static_assert(W % 2 == 0, "word rows");
+  const uint32_t *sw = reinterpret_cast<const uint32_t *>(src);
+  const unsigned short *sh = reinterpret_cast<const unsigned short *>(src);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < T; i += THREADS) {
+    const int x = i % WW, y = (i / WW) % H, c = (i / (WW * H)) % CC, img = i / (WW * H * CC);
+    uint32_t v = 0;
+    if (img < n) {
+      const size_t o = (((size_t)img * CT + c0 + c) * H + y) * WW + x;
+      v = words ? __ldg(sw + o) : (uint32_t)__ldg(sh + 2 * o) | (uint32_t)__ldg(sh + 2 * o + 1) << 16;
+    }
+    reinterpret_cast<uint32_t *>(s)[((c * NI + img) * plane_n(L) + (y + P) * plane_w(L)) / 2 + x + 1] = v;
+  }
+}
+
+// ---------------------------------------------------------------- forward --
+// A conv layer on the block's images: units of MT m tiles x NT n tiles of 8
+// output pixels, one warp each. The result goes to the activation tensor and,
+// but for conv4, to the next layer's planes.
+template <int L, int NI, int MT, int NT>
+__device__ __forceinline__ void conv_fwd_layer(const bf16 *__restrict__ s_in,
+                                               const ushort4 *__restrict__ tab,
+                                               const uint4 *__restrict__ fw,
+                                               const float *__restrict__ bias,
+                                               bf16 *__restrict__ s_out, bf16 *__restrict__ out,
+                                               int nimg) {
+  constexpr ConvSpec c = kConv[L];
+  constexpr int HW = c.ho * c.wo, KS = fw_ks(L), PL = plane_n(L), PW = plane_w(L);
+  constexpr int TILES = (NI * HW + 7) / 8, NU = (TILES + NT - 1) / NT, MU = fw_mt(L) / MT;
+  static_assert(fw_mt(L) % MT == 0 && HW % 2 == 0, "unit shape");
+  const unsigned short *in = reinterpret_cast<const unsigned short *>(s_in);
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int u = threadIdx.x >> 5; u < NU * MU; u += kTrWarps) {
+    const int mu = u % MU, nu = u / MU;
+    int nb[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int n = min((nu * NT + j) * 8 + g, NI * HW - 1);  // (pixels past the end: not stored)
+      const int img = n / HW, p = n % HW;
+      nb[j] = img * PL + (p / c.wo) * c.s * PW + (p % c.wo) * c.s + 2 - c.p;
+    }
+    float acc[MT][NT][4] = {};
+    const uint4 *fa = fw + ((size_t)(fw_first(L) + mu * MT * KS)) * 32 + lane;
+    // the next step's weights are on their way while this one's are used
+    uint4 nxt[2][MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      nxt[0][m] = __ldg(fa + (size_t)m * KS * 32);
+      nxt[1][m] = __ldg(fa + ((size_t)m * KS + (KS > 1 ? 1 : 0)) * 32);
+    }
+#pragma unroll 2
+    for (int s = 0; s < KS; ++s) {
+      uint4 a[MT];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        a[m] = nxt[0][m];
+        nxt[0][m] = nxt[1][m];
+        if (s + 2 < KS) nxt[1][m] = __ldg(fa + ((size_t)m * KS + s + 2) * 32);
+      }
+      const ushort4 o = tab[s * 4 + t];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const unsigned short *q = in + nb[j];
+        uint32_t b0 = (uint32_t)q[o.x] | (uint32_t)q[o.y] << 16;
+        uint32_t b1 = (uint32_t)q[o.z] | (uint32_t)q[o.w] << 16;
+        if (fw_k(L) % 16 != 0 && s == KS - 1) {  // k beyond K reads as 0
+          constexpr int r = fw_k(L) % 16;
+          if (2 * t >= r) b0 = 0u;
+          if (2 * t + 8 >= r) b1 = 0u;
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m) mma_bf16(acc[m][j], a[m], b0, b1);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int co = (mu * MT + m) * 16 + g + 8 * h;
+        const float b = __ldg(bias + co);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const int n = (nu * NT + j) * 8 + 2 * t, img = n / HW, p = n % HW;
+          if (n >= NI * HW || img >= nimg) continue;
+          const bf16 v0 = __float2bfloat16_rn(fmaxf(acc[m][j][2 * h] + b, 0.f));
+          const bf16 v1 = __float2bfloat16_rn(fmaxf(acc[m][j][2 * h + 1] + b, 0.f));
+          *reinterpret_cast<__nv_bfloat162 *>(out + ((size_t)img * c.co + co) * HW + p) =
+              __nv_bfloat162(v0, v1);
+          if constexpr (L < 3) {
+            bf16 *d = s_out + (co * NI + img) * plane_n(L + 1) + 2;
+            d[(p / c.wo + kConv[L + 1].p) * plane_w(L + 1) + p % c.wo] = v0;
+            d[((p + 1) / c.wo + kConv[L + 1].p) * plane_w(L + 1) + (p + 1) % c.wo] = v1;
+          }
+        }
+      }
+  }
+}
+
+template <int NI>
+struct FwdSmem {
+  alignas(16) bf16 in[2 * NI * plane_n(0)];
+  alignas(16) bf16 a1[16 * NI * plane_n(1)];
+  alignas(16) bf16 a2[32 * NI * plane_n(2)];
+  alignas(16) bf16 a3[64 * NI * plane_n(3)];
+  alignas(16) ushort4 t0[fw_ks(0) * 4], t1[fw_ks(1) * 4], t2[fw_ks(2) * 4], t3[fw_ks(3) * 4];
+};
+static_assert(sizeof(FwdSmem<2>) <= 227 * 1024 && sizeof(FwdSmem<1>) <= 113 * 1024, "shared memory");
+
+// conv1..conv4 of NI images at a time, one block; the activations between the
+// layers stay in shared memory (and are written out for the backward pass).
+// NI = 2 fills conv4's tiles of 8 pixels (40 = 5 x 8, against 20 in 24) and
+// halves the weight reads; NI = 1 gives small batches a block an image. At
+// batch 256 the 128 blocks of two images run in one wave.
+template <int NI>
+__global__ void __launch_bounds__(kTrThreads) k_conv_fwd(const bf16 *__restrict__ in,
+                                                         const uint4 *__restrict__ fw,
+                                                         const float *__restrict__ pm, int batch,
+                                                         bool words, bf16 *__restrict__ a1,
+                                                         bf16 *__restrict__ a2,
+                                                         bf16 *__restrict__ a3,
+                                                         bf16 *__restrict__ a4) {
+  extern __shared__ __align__(16) unsigned char s_train[];
+  FwdSmem<NI> &S = *reinterpret_cast<FwdSmem<NI> *>(s_train);
+  uint4 *z = reinterpret_cast<uint4 *>(s_train);
+  for (int i = threadIdx.x; i < (int)(sizeof(FwdSmem<NI>) / 16); i += kTrThreads)
+    z[i] = make_uint4(0u, 0u, 0u, 0u);  // the planes' borders stay zero
+  __syncthreads();
+  fill_taps<0, NI>(S.t0);
+  fill_taps<1, NI>(S.t1);
+  fill_taps<2, NI>(S.t2);
+  fill_taps<3, NI>(S.t3);
+  for (int b = blockIdx.x * NI; b < batch; b += gridDim.x * NI) {
+    const int n = min(NI, batch - b);
+    stage_images<0, NI, 2, kTrThreads>(in + (size_t)b * kActIn, n, 0, S.in, words);
+    __syncthreads();
+    conv_fwd_layer<0, NI, 1, 4>(S.in, S.t0, fw, pm + kOffB0, S.a1, a1 + b * kAct0, n);
+    __syncthreads();
+    conv_fwd_layer<1, NI, 2, NI == 2 ? 5 : 3>(S.a1, S.t1, fw, pm + kOffB1, S.a2,
+                                              a2 + b * kAct1, n);
+    __syncthreads();
+    conv_fwd_layer<2, NI, 1, NI == 2 ? 5 : 3>(S.a2, S.t2, fw, pm + kOffB2, S.a3,
+                                              a3 + b * kAct2, n);
+    __syncthreads();
+    conv_fwd_layer<3, NI, 1, NI == 2 ? 3 : 2>(S.a3, S.t3, fw, pm + kOffB3, nullptr,
+                                              a4 + b * kAct3, n);
+  }
+}
+
+// FC1 and FC2 of 8 pairs, one block of 10 warps (a warp an m tile of FC1's
+// 160 outputs), and, when `target` is given, the loss and the gradient at
+// FC1's output (masked by its ReLU and rounded to TF32, as its readers take
+// it). Bound by the chain of 160 k steps: the packed weights are requested 8
+// steps ahead. With `given`, f1 and out come from another kernel (small
+// batches).
+constexpr int kHeadThreads = 320, kHeadN = 8, kHeadPad = 8;
+__global__ void __launch_bounds__(kHeadThreads)
+    k_head(const bf16 *__restrict__ a4, const uint4 *__restrict__ fw, const bf16 *__restrict__ pw,
+           const float *__restrict__ pm, int batch, bool given, bf16 *__restrict__ f1,
+           float *__restrict__ out, const float *__restrict__ target, const float *__restrict__ wk,
+           float *__restrict__ gout, float *__restrict__ gf1, float *__restrict__ loss) {
+  __shared__ alignas(16) bf16 s_a4[kHeadN][kF1In + kHeadPad];
+  __shared__ alignas(16) bf16 s_f1[kHeadN][kF1Out + kHeadPad];
+  __shared__ float s_out[kHeadN][8], s_g[kHeadN][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int b0 = blockIdx.x * kHeadN, nb = min(kHeadN, batch - b0);
+  if (!given) {
+    constexpr int KS = fw_ks(4), AHEAD = 8;
+    static_assert(KS % AHEAD == 0 && kF1In % 8 == 0 && fw_mt(4) * 32 == kHeadThreads, "FC1 shape");
+    const uint4 *fa = fw + ((size_t)fw_first(4) + warp * KS) * 32 + lane;
+    uint4 a[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) a[i] = __ldg(fa + i * 32);
+    const uint4 *src = reinterpret_cast<const uint4 *>(a4 + (size_t)b0 * kF1In);
+    for (int i = threadIdx.x; i < kHeadN * (kF1In / 8); i += kHeadThreads) {
+      const int r = i / (kF1In / 8), q = i % (kF1In / 8);
+      *reinterpret_cast<uint4 *>(&s_a4[r][8 * q]) =
+          r < nb ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    float c[4] = {};
+    const bf16 *row = &s_a4[g][2 * t];
+    for (int s = 0; s < KS; s += AHEAD)
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const uint4 w = a[i];
+        if (s + i + AHEAD < KS) a[i] = __ldg(fa + (s + i + AHEAD) * 32);
+        const uint32_t q0 = *reinterpret_cast<const uint32_t *>(row + (s + i) * 16);
+        const uint32_t q1 = *reinterpret_cast<const uint32_t *>(row + (s + i) * 16 + 8);
+        mma_bf16(c, w, q0, q1);
+      }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = warp * 16 + g + (r >= 2 ? 8 : 0), n = 2 * t + (r & 1);
+      const bf16 v = __float2bfloat16_rn(fmaxf(c[r] + __ldg(pm + kOffBF1 + m), 0.f));
+      s_f1[n][m] = v;
+      if (n < nb) f1[(size_t)(b0 + n) * kF1Out + m] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      float d[4] = {};
+      const uint4 *f2 = fw + (size_t)fw_first(5) * 32 + lane;
+#pragma unroll
+      for (int s = 0; s < fw_ks(5); ++s)
+        mma_bf16(d, __ldg(f2 + s * 32), *reinterpret_cast<const uint32_t *>(&s_f1[g][s * 16 + 2 * t]),
+                 *reinterpret_cast<const uint32_t *>(&s_f1[g][s * 16 + 8 + 2 * t]));
+      if (g < kF2Out) {
+        const float bias = __ldg(pm + kOffBF2 + g);
+        s_out[2 * t][g] = d[0] + bias;
+        s_out[2 * t + 1][g] = d[1] + bias;
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < kHeadN * kF1Out; i += kHeadThreads) {
+      const int r = i / kF1Out, m = i % kF1Out;
+      s_f1[r][m] = r < nb ? f1[(size_t)(b0 + r) * kF1Out + m] : __float2bfloat16_rn(0.f);
+    }
+    if (threadIdx.x < kHeadN * kF2Out) {
+      const int r = threadIdx.x / kF2Out, m = threadIdx.x % kF2Out;
+      s_out[r][m] = r < nb ? out[(size_t)(b0 + r) * kF2Out + m] : 0.f;
+    }
+  }
+  __syncthreads();
+  if (!given && threadIdx.x < nb * kF2Out)
+    out[(size_t)b0 * kF2Out + threadIdx.x] = s_out[threadIdx.x / kF2Out][threadIdx.x % kF2Out];
+  if (!target) return;
+  // mean over the batch of sum_k wk (out - target)^2 and its gradient
+  if (threadIdx.x < kHeadN) {
+    const int r = threadIdx.x;
+    float l = 0.f;
+    for (int k = 0; k < 8; ++k) {
+      float gk = 0.f;
+      if (r < nb && k < kF2Out) {
+        const float e = s_out[r][k] - target[(size_t)(b0 + r) * kF2Out + k];
+        l = fmaf(wk[k] * e, e, l);
+        gk = 2.f * wk[k] * e / (float)batch;
+        gout[(size_t)(b0 + r) * kF2Out + k] = gk;
+      }
+      s_g[r][k] = to_tf32(gk);
+    }
+    if (r < nb) loss[b0 + r] = l;
+  }
+  __syncthreads();
+  // FC2's input gradient: one k8 step (6 outputs and two zeros)
+  {
+    const bf16 *w2 = pw + kOffF2;
+    auto w = [&](int k, int i) { return k < kF2Out ? bf(w2[k * kF1Out + i]) : 0.f; };
+    const int m = warp * 16 + g;
+    float c[4] = {};
+    mma_tf32(c, w(t, m), w(t, m + 8), w(t + 4, m), w(t + 4, m + 8), s_g[g][t], s_g[g][t + 4]);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = m + (r >= 2 ? 8 : 0), n = 2 * t + (r & 1);
+      if (n < nb)
+        gf1[(size_t)(b0 + n) * kF1Out + i] = bf(s_f1[n][i]) > 0.f ? to_tf32(c[r]) : 0.f;
+    }
+  }
+}
+
+// --------------------------------------------------- FC backward ----------
+// Blocks [0, dgrad_blocks): FC1's input gradient g4 = W1^T gf1 (masked by
+// conv4's ReLU, rounded to TF32), 8 m tiles (a warp each) x 64 pairs a block.
+// Then kF1WBlocks blocks: FC1's weight gradient, 64 input columns x all 160
+// rows over the whole batch, 10 warps; and one block with both layers' biases
+// and FC2's weights. All three read gf1 only, so they share one launch.
+constexpr int kFcThreads = 320, kFcPairs = 64, kFcGPad = 4;
+constexpr int kF1WCols = 64, kF1WBlocks = kF1In / kF1WCols;
+static_assert(kF1WBlocks * kF1WCols == kF1In && kF1In % 128 == 0, "FC1 column blocks");
+__global__ void __launch_bounds__(kFcThreads)
+    k_fc_bwd(const float *__restrict__ gf1, const float *__restrict__ gout,
+             const bf16 *__restrict__ a4, const bf16 *__restrict__ f1, const bf16 *__restrict__ pw,
+             int batch, int dgrad_blocks, float *__restrict__ g4, float *__restrict__ grad) {
+  __shared__ float s_g[kFcPairs][kF1Out + kFcGPad];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  int blk = blockIdx.x;
+  if (blk < dgrad_blocks) {
+    const int mb = blk % (kF1In / 128), b0 = (blk / (kF1In / 128)) * kFcPairs;
+    const int nb = min(kFcPairs, batch - b0);
+    for (int i = threadIdx.x; i < kFcPairs * kF1Out; i += kFcThreads) {
+      const int r = i / kF1Out, j = i % kF1Out;
+      s_g[r][j] = r < nb ? __ldg(gf1 + (size_t)(b0 + r) * kF1Out + j) : 0.f;
+    }
+    __syncthreads();
+    if (warp >= 8) return;
+    const int m = (mb * 8 + warp) * 16 + g;
+    const bf16 *w1 = pw + kOffF1 + m;
+    float c[kFcPairs / 8][4] = {};
+#pragma unroll 5
+    for (int s = 0; s < kF1Out / 8; ++s) {
+      const bf16 *w = w1 + (size_t)(s * 8 + t) * kF1In;
+      const float x0 = bf(w[0]), x1 = bf(w[8]), x2 = bf(w[4 * kF1In]), x3 = bf(w[4 * kF1In + 8]);
+#pragma unroll
+      for (int j = 0; j < kFcPairs / 8; ++j)
+        mma_tf32(c[j], x0, x1, x2, x3, s_g[j * 8 + g][s * 8 + t], s_g[j * 8 + g][s * 8 + t + 4]);
+    }
+#pragma unroll
+    for (int j = 0; j < kFcPairs / 8; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = m + (r >= 2 ? 8 : 0), n = j * 8 + 2 * t + (r & 1);
+        if (n >= nb) continue;
+        const size_t o = (size_t)(b0 + n) * kF1In + i;
+        g4[o] = bf(a4[o]) > 0.f ? to_tf32(c[j][r]) : 0.f;
+      }
+    return;
+  }
+  blk -= dgrad_blocks;
+  if (blk < kF1WBlocks) {
+    // m = j (one m tile a warp), n = i, k = pair
+    const int m = warp * 16 + g, i0 = blk * kF1WCols;
+    float c[kF1WCols / 8][4] = {};
+#pragma unroll 4
+    for (int k0 = 0; k0 < batch; k0 += 8) {
+      const int ka = k0 + t, kb = k0 + t + 4;
+      const bool va = ka < batch, vb = kb < batch;
+      const float *ga = gf1 + (size_t)(va ? ka : 0) * kF1Out + m, *gb = gf1 + (size_t)(vb ? kb : 0) * kF1Out + m;
+      const float x0 = va ? __ldg(ga) : 0.f, x1 = va ? __ldg(ga + 8) : 0.f;
+      const float x2 = vb ? __ldg(gb) : 0.f, x3 = vb ? __ldg(gb + 8) : 0.f;
+      const bf16 *pa = a4 + (size_t)(va ? ka : 0) * kF1In + i0 + g, *pb = a4 + (size_t)(vb ? kb : 0) * kF1In + i0 + g;
+#pragma unroll
+      for (int j = 0; j < kF1WCols / 8; ++j)
+        mma_tf32(c[j], x0, x1, x2, x3, va ? bf(pa[8 * j]) : 0.f, vb ? bf(pb[8 * j]) : 0.f);
+    }
+#pragma unroll
+    for (int j = 0; j < kF1WCols / 8; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        grad[kOffF1 + (size_t)(m + (r >= 2 ? 8 : 0)) * kF1In + i0 + j * 8 + 2 * t + (r & 1)] = c[j][r];
+    return;
+  }
+  blk -= kF1WBlocks;
+  // FC2's weights (a warp an m16 x n16 tile; 6 of 16 rows are live)
+  if (blk == 0) {
+    const int i0 = warp * 16;
+    float c[2][4] = {};
+    for (int k0 = 0; k0 < batch; k0 += 8) {
+      const int ka = k0 + t, kb = k0 + t + 4;
+      const bool va = ka < batch, vb = kb < batch;
+      const float x0 = va && g < kF2Out ? to_tf32(__ldg(gout + (size_t)ka * kF2Out + g)) : 0.f;
+      const float x2 = vb && g < kF2Out ? to_tf32(__ldg(gout + (size_t)kb * kF2Out + g)) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        mma_tf32(c[j], x0, 0.f, x2, 0.f, va ? bf(f1[(size_t)ka * kF1Out + i0 + 8 * j + g]) : 0.f,
+                 vb ? bf(f1[(size_t)kb * kF1Out + i0 + 8 * j + g]) : 0.f);
+    }
+    if (g < kF2Out)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        grad[kOffF2 + g * kF1Out + i0 + 8 * j + 2 * t] = c[j][0];
+        grad[kOffF2 + g * kF1Out + i0 + 8 * j + 2 * t + 1] = c[j][1];
+      }
+    return;
+  }
+  // the bias gradients: blocks of 32 columns, 10 warps over the pairs
+  const int j = (blk - 1) * 32 + lane;
+  float s = 0.f;
+  if (j < kF1Out)
+    for (int k = warp; k < batch; k += kFcThreads / 32) s += __ldg(gf1 + (size_t)k * kF1Out + j);
+  else if (j < kF1Out + kF2Out)
+    for (int k = warp; k < batch; k += kFcThreads / 32)
+      s += to_tf32(__ldg(gout + (size_t)k * kF2Out + j - kF1Out));
+  s_g[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && j < kF1Out + kF2Out) {
+    float a = 0.f;
+    for (int w = 0; w < kFcThreads / 32; ++w) a += s_g[w][lane];
+    grad[j < kF1Out ? kOffBF1 + j : kOffBF2 + j - kF1Out] = a;
+  }
+}
+constexpr int kFcBiasBlocks = (kF1Out + kF2Out + 31) / 32;
+
+// ------------------------------------------------ conv input gradients --
+// Layer L's input gradient from the gradient at its (masked) output, stride 2:
+// input pixel (iy, ix) = (2r + py, 2c + px) takes tap (ky, kx) from output
+// pixel (r + dy, c + dx) with, per axis, parity 0: tap 1, offset 0; parity 1:
+// tap 0, offset 1 and tap 2, offset 0; the other taps contribute zeros. The n
+// tiles hold pixels of one parity class, so a tap's offset is the same for all
+// of them; a tap that does not reach the class points into a plane of zeros
+// (its products stay in the sum, in their place). Gradient planes:
+// [co][image][ho + 1][wo + 1], the last row and column zero, and one zero
+// plane after the last channel.
+constexpr int gplane_w(int l) { return kConv[l].wo + 1; }
+constexpr int gplane_n(int l) { return (kConv[l].ho + 1) * (kConv[l].wo + 1); }
+template <int L, int NI>
+__device__ __forceinline__ void fill_bwd_taps(ushort2 *tab) {
+  static_assert((kConv[L].co + 1) * NI * gplane_n(L) < 65536, "16-bit offsets");
+  auto offset = [](int cls, int k) {
+    const int co = k / 9, ky = (k % 9) / 3, kx = k % 3, py = cls >> 1, px = cls & 1;
+    if ((py ? ky == 1 : ky != 1) || (px ? kx == 1 : kx != 1)) return kConv[L].co * NI * gplane_n(L);
+    return co * NI * gplane_n(L) + (py && ky == 0 ? gplane_w(L) : 0) + (px && kx == 0 ? 1 : 0);
+  };
+  for (int i = threadIdx.x; i < 4 * bw_ks(L) * 4; i += kTrThreads) {
+    const int t = i & 3, s = (i >> 2) % bw_ks(L), cls = (i >> 2) / bw_ks(L);
+    tab[i] = make_ushort2(offset(cls, s * 8 + t), offset(cls, s * 8 + t + 4));
+  }
+}
+
+template <int L, int NI, int MT, int NT>
+__device__ __forceinline__ void conv_bwd_layer(const float *__restrict__ s_g,
+                                               const ushort2 *__restrict__ tab,
+                                               const uint2 *__restrict__ bw,
+                                               const bf16 *__restrict__ act,
+                                               float *__restrict__ s_out, float *__restrict__ gin,
+                                               int nimg) {
+  constexpr ConvSpec c = kConv[L];
+  constexpr int KS = bw_ks(L), PL = gplane_n(L), PW = gplane_w(L), MU = bw_mt(L) / MT;
+  constexpr int MAXPX = NI * ((c.hi + 1) / 2) * ((c.wi + 1) / 2);
+  constexpr int NU = ((MAXPX + 7) / 8 + NT - 1) / NT;
+  static_assert(c.wi % 2 == 0 && bw_mt(L) % MT == 0 && KS % 4 == 0, "unit shape");
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int u = threadIdx.x >> 5; u < 4 * NU * MU; u += kTrWarps) {
+    const int mu = u % MU, cls = (u / MU) & 3, nu = u / (4 * MU);
+    const int py = cls >> 1, px = cls & 1;
+    const int nc = c.wi / 2, cnt = ((c.hi + 1 - py) / 2) * nc;
+    if (nu * NT * 8 >= NI * cnt) continue;
+    int nb[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int n = min((nu * NT + j) * 8 + g, NI * cnt - 1), img = n / cnt, p = n % cnt;
+      nb[j] = img * PL + (p / nc) * PW + p % nc;
+    }
+    float acc[MT][NT][4] = {};
+    const uint2 *fa = bw + ((size_t)(bw_first(L) + mu * MT * KS)) * 32 + lane;
+    const ushort2 *ct = tab + cls * KS * 4 + t;
+    // four steps of weights ahead
+    uint2 nxt[4][MT];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < MT; ++m) nxt[i][m] = __ldg(fa + (m * KS + i) * 32);
+    for (int s = 0; s < KS; s += 4)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint2 a[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          a[m] = nxt[i][m];
+          if (s + i + 4 < KS) nxt[i][m] = __ldg(fa + (m * KS + s + i + 4) * 32);
+        }
+        const ushort2 o = ct[(s + i) * 4];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const float b0 = s_g[nb[j] + o.x], b1 = s_g[nb[j] + o.y];
+#pragma unroll
+          for (int m = 0; m < MT; ++m)
+            mma_tf32(acc[m][j], bits_f(a[m].x & 0xffffu), __uint_as_float(a[m].x & 0xffff0000u),
+                     bits_f(a[m].y & 0xffffu), __uint_as_float(a[m].y & 0xffff0000u), b0, b1);
+        }
+      }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int n = (nu * NT + j) * 8 + 2 * t + h, img = n / cnt, p = n % cnt;
+        if (n >= NI * cnt || img >= nimg) continue;
+        const int y = 2 * (p / nc) + py, x = 2 * (p % nc) + px;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int ci = (mu * MT + m) * 16 + g + 8 * r;
+            const size_t o = ((size_t)img * c.ci + ci) * (c.hi * c.wi) + y * c.wi + x;
+            const float v = bf(act[o]) > 0.f ? to_tf32(acc[m][j][2 * r + h]) : 0.f;
+            gin[o] = v;
+            if constexpr (L > 1) s_out[(ci * NI + img) * gplane_n(L - 1) + y * gplane_w(L - 1) + x] = v;
+          }
+      }
+  }
+}
+
+template <int NI>
+struct BwdSmem {
+  alignas(16) float g4[129 * NI * gplane_n(3)];
+  alignas(16) float g3[65 * NI * gplane_n(2)];
+  alignas(16) float g2[33 * NI * gplane_n(1)];
+  alignas(16) ushort2 t3[4 * bw_ks(3) * 4], t2[4 * bw_ks(2) * 4], t1[4 * bw_ks(1) * 4];
+};
+static_assert(sizeof(BwdSmem<2>) <= 227 * 1024 && sizeof(BwdSmem<1>) <= 113 * 1024, "shared memory");
+
+// The input gradients of conv4, conv3 and conv2 of NI images at a time, one
+// block; each is masked by the ReLU below it and rounded to TF32, which is
+// how the next layer and the weight gradients read it. Bound by the tensor
+// pipe's TF32 rate and the shared-memory gathers that feed it.
+template <int NI>
+__global__ void __launch_bounds__(kTrThreads) k_conv_dgrad(const float *__restrict__ g4,
+                                                           const uint2 *__restrict__ bw, int batch,
+                                                           const bf16 *__restrict__ a1,
+                                                           const bf16 *__restrict__ a2,
+                                                           const bf16 *__restrict__ a3,
+                                                           float *__restrict__ g1,
+                                                           float *__restrict__ g2,
+                                                           float *__restrict__ g3) {
+  extern __shared__ __align__(16) unsigned char s_train[];
+  BwdSmem<NI> &S = *reinterpret_cast<BwdSmem<NI> *>(s_train);
+  uint4 *z = reinterpret_cast<uint4 *>(s_train);
+  for (int i = threadIdx.x; i < (int)(sizeof(BwdSmem<NI>) / 16); i += kTrThreads)
+    z[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  fill_bwd_taps<3, NI>(S.t3);
+  fill_bwd_taps<2, NI>(S.t2);
+  fill_bwd_taps<1, NI>(S.t1);
+  for (int b = blockIdx.x * NI; b < batch; b += gridDim.x * NI) {
+    const int n = min(NI, batch - b);
+    constexpr int HW = kConv[3].ho * kConv[3].wo;
+    for (int i = threadIdx.x; i < NI * (int)kAct3; i += kTrThreads) {
+      const int img = i / (int)kAct3, co = (i / HW) % 128, p = i % HW;
+      S.g4[(co * NI + img) * gplane_n(3) + (p / kConv[3].wo) * gplane_w(3) + p % kConv[3].wo] =
+          img < n ? __ldg(g4 + b * kAct3 + i) : 0.f;
+    }
+    __syncthreads();
+    conv_bwd_layer<3, NI, 1, NI == 2 ? 5 : 3>(S.g4, S.t3, bw, a3 + b * kAct2, S.g3,
+                                              g3 + b * kAct2, n);
+    __syncthreads();
+    conv_bwd_layer<2, NI, 2, NI == 2 ? 5 : 3>(S.g3, S.t2, bw, a2 + b * kAct1, S.g2,
+                                              g2 + b * kAct1, n);
+    __syncthreads();
+    conv_bwd_layer<1, NI, 1, NI == 2 ? 5 : 5>(S.g2, S.t1, bw, a1 + b * kAct0, nullptr,
+                                              g1 + b * kAct0, n);
+  }
+}
+
+// ----------------------------------------------- conv weight gradients --
+// m = co, n = (ci, ky, kx), k = output pixel over the block's images. The
+// layer's input sits in padded planes (double-buffered by cp.async words), so
+// an operand is at pixel offset + tap offset; the gradient operand, used by
+// one warp or a few, comes straight from memory one k step ahead. Warps split
+// the tile as MG m tiles x NG groups of NTW n tiles x KG shares of the k
+// steps. One launch holds the four layers (block ranges): their blocks fill
+// the SMs together. Partial sums over a block's images go to `part`; the
+// reduction adds them in block order, so a run is reproducible bit for bit.
+template <int L> struct WgCfg;
+template <> struct WgCfg<0> { static constexpr int CC = 2, NI = 1, MG = 1, NG = 1, KG = 16, NTW = 7; };
+template <> struct WgCfg<1> { static constexpr int CC = 16, NI = 2, MG = 2, NG = 2, KG = 4, NTW = 9; };
+template <> struct WgCfg<2> { static constexpr int CC = 32, NI = 2, MG = 4, NG = 4, KG = 1, NTW = 9; };
+template <> struct WgCfg<3> { static constexpr int CC = 16, NI = 4, MG = 8, NG = 2, KG = 1, NTW = 9; };
+
+template <int L>
+struct WgSmem {
+  using C = WgCfg<L>;
+  static constexpr int K = C::NI * kConv[L].ho * kConv[L].wo;
+  static_assert(K % 8 == 0, "whole k steps");
+  alignas(16) bf16 x[2][C::CC * C::NI * plane_n(L)];
+  int2 kinfo[K];  // per k: pixel offset in the planes, offset in the gradient
+  float red[C::KG > 1 ? (C::KG - 1) * C::MG * C::NG * (C::NTW * 4 + 2) * 32 : 1];
+};
+constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
+constexpr size_t kWgSmem = cmax(cmax(sizeof(WgSmem<0>), sizeof(WgSmem<1>)),
+                                cmax(sizeof(WgSmem<2>), sizeof(WgSmem<3>)));
+static_assert(kWgSmem <= 227 * 1024, "shared memory");
+constexpr int wg_chunks(int l) { return l == 3 ? 4 : 1; }  // conv4's input channels, 16 a block
+constexpr int wg_ni(int l) { return l == 0 ? 1 : l == 3 ? 4 : 2; }
+constexpr int wg_size(int l) { return kConv[l].co * (kConv[l].ci * kConv[l].k * kConv[l].k + 1); }
+
+// How many blocks share a layer's images (slices), for at most about a wave
+// of 148 blocks in all: the layers' multiply-adds at full batch are alike
+// (conv1 78 %), conv4's slices come in chunks of 4.
+struct WgPlan {
+  int slices[4];
+  int first[5];      // block ranges
+  long part[4];      // offsets of the layers' partial sums, floats
+  long total;
+};
+inline WgPlan wg_plan(int batch) {
+  constexpr int kWant[4] = {32, 38, 38, 10};
+  WgPlan p;
+  p.first[0] = 0;
+  p.total = 0;
+  for (int l = 0; l < 4; ++l) {
+    const int groups = (batch + wg_ni(l) - 1) / wg_ni(l);
+    p.slices[l] = groups < kWant[l] ? groups : kWant[l];
+    p.first[l + 1] = p.first[l] + p.slices[l] * wg_chunks(l);
+    p.part[l] = p.total;
+    p.total += (long)p.slices[l] * wg_size(l);
+  }
+  return p;
+}
+
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, bool live) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  const int n = live ? 4 : 0;  // (0 source bytes: the word is zeroed)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
+}
+
+template <int L>
+__device__ __forceinline__ void wg_stage(const bf16 *__restrict__ src, int n, int c0, bf16 *s,
+                                         bool words) {
+  using C = WgCfg<L>;
+  if (!words) {
+    stage_images<L, C::NI, C::CC, kTrThreads>(src, n, c0, s, false);
+    return;
+  }
+  constexpr int H = kConv[L].hi, WW = kConv[L].wi / 2, CT = kConv[L].ci, P = kConv[L].p;
+  constexpr int T = C::CC * C::NI * H * WW;
+  const uint32_t *sw = reinterpret_cast<const uint32_t *>(src);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < T; i += kTrThreads) {
+    const int x = i % WW, y = (i / WW) % H, c = (i / (WW * H)) % C::CC, img = i / (WW * H * C::CC);
+    const bool live = img < n;
+    const size_t o = live ? (((size_t)img * CT + c0 + c) * H + y) * WW + x : 0;
+    cp_async4(reinterpret_cast<uint32_t *>(s) +
+                  ((c * C::NI + img) * plane_n(L) + (y + P) * plane_w(L)) / 2 + x + 1,
+              sw + o, live);
+  }
+}
+
+template <int L>
+__device__ __forceinline__ void conv_wgrad(const bf16 *__restrict__ in, const float *__restrict__ gr,
+                                           int batch, int slice, int slices, int chunk, bool words,
+                                           float *__restrict__ part) {
+  using C = WgCfg<L>;
+  constexpr ConvSpec c = kConv[L];
+  constexpr int HW = c.ho * c.wo, KK = c.k * c.k, N = c.ci * KK, NC = C::CC * KK;
+  constexpr int K = WgSmem<L>::K, STEPS = K / 8;
+  static_assert(C::MG * 16 == c.co && C::MG * C::NG * C::KG == kTrWarps &&
+                    C::NG * C::NTW * 8 >= NC, "warp split");
+  extern __shared__ __align__(16) unsigned char s_train[];
+  WgSmem<L> &S = *reinterpret_cast<WgSmem<L> *>(s_train);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int mg = warp % C::MG, ng = (warp / C::MG) % C::NG, kg = warp / (C::MG * C::NG);
+  for (int i = threadIdx.x; i < (int)(sizeof(S.x) / 4); i += kTrThreads)
+    reinterpret_cast<uint32_t *>(&S.x[0][0])[i] = 0u;
+  for (int k = threadIdx.x; k < K; k += kTrThreads) {
+    const int img = k / HW, p = k % HW;
+    S.kinfo[k] = make_int2(img * plane_n(L) + (p / c.wo) * c.s * plane_w(L) + (p % c.wo) * c.s + 2 - c.p,
+                           img * c.co * HW + p);
+  }
+  int off[C::NTW];  // this lane's tap of each n tile (a column past the end repeats tap 0, not stored)
+#pragma unroll
+  for (int j = 0; j < C::NTW; ++j) {
+    const int n = (ng * C::NTW + j) * 8 + g, q = n < NC ? n : 0;
+    off[j] = (q / KK) * C::NI * plane_n(L) + ((q % KK) / c.k) * plane_w(L) + q % c.k;
+  }
+  float acc[C::NTW][4] = {};
+  float bs0 = 0.f, bs1 = 0.f;
+  const int groups = (batch + C::NI - 1) / C::NI;
+  const int c0 = chunk * C::CC;
+  __syncthreads();
+  int buf = 0;
+  {
+    const int b = slice * C::NI;
+    wg_stage<L>(in + (size_t)b * c.ci * c.hi * c.wi, min(C::NI, batch - b), c0, S.x[0], words);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int gi = slice; gi < groups; gi += slices, buf ^= 1) {
+    const int b = gi * C::NI, n = min(C::NI, batch - b);
+    if (gi + slices < groups) {
+      const int b2 = (gi + slices) * C::NI;
+      wg_stage<L>(in + (size_t)b2 * c.ci * c.hi * c.wi, min(C::NI, batch - b2), c0, S.x[buf ^ 1], words);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    const unsigned short *x = reinterpret_cast<const unsigned short *>(S.x[buf]);
+    const float *ga = gr + (size_t)b * c.co * HW + (mg * 16 + g) * HW;
+    const int klive = n * HW;
+    // the gradient operand of a step (zero past the last image)
+    auto load_a = [&](int s, int &pa, int &pb, float (&a)[4]) {
+      const int ka = s * 8 + t, kb = ka + 4;
+      const int2 ia = S.kinfo[ka], ib = S.kinfo[kb];
+      pa = ia.x;
+      pb = ib.x;
+      const bool va = ka < klive, vb = kb < klive;
+      a[0] = va ? __ldg(ga + ia.y) : 0.f;
+      a[1] = va ? __ldg(ga + ia.y + 8 * HW) : 0.f;
+      a[2] = vb ? __ldg(ga + ib.y) : 0.f;
+      a[3] = vb ? __ldg(ga + ib.y + 8 * HW) : 0.f;
+    };
+    int pa = 0, pb = 0;
+    float a[4] = {};
+    if (kg < STEPS) load_a(kg, pa, pb, a);
+#pragma unroll 2
+    for (int s = kg; s < STEPS; s += C::KG) {
+      int na = 0, nb = 0;
+      float an[4] = {};
+      if (s + C::KG < STEPS) load_a(s + C::KG, na, nb, an);
+#pragma unroll
+      for (int j = 0; j < C::NTW; ++j)
+        mma_tf32(acc[j], a[0], a[1], a[2], a[3], bits_f(x[pa + off[j]]), bits_f(x[pb + off[j]]));
+      if (ng == 0) {
+        bs0 += a[0] + a[2];
+        bs1 += a[1] + a[3];
+      }
+      pa = na;
+      pb = nb;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = an[i];
+    }
+    __syncthreads();
+  }
+  // the k shares of a tile, added in order
+  if constexpr (C::KG > 1) {
+    constexpr int V = C::NTW * 4 + 2;
+    const int q = mg + C::MG * ng;
+    if (kg > 0) {
+      float *r = S.red + ((size_t)((kg - 1) * C::MG * C::NG + q) * V) * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < C::NTW; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[(4 * j + i) * 32] = acc[j][i];
+      r[(V - 2) * 32] = bs0;
+      r[(V - 1) * 32] = bs1;
+    }
+    __syncthreads();
+    if (kg > 0) return;
+    for (int k = 1; k < C::KG; ++k) {
+      const float *r = S.red + ((size_t)((k - 1) * C::MG * C::NG + q) * V) * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < C::NTW; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] += r[(4 * j + i) * 32];
+      bs0 += r[(V - 2) * 32];
+      bs1 += r[(V - 1) * 32];
+    }
+  }
+  float *dst = part + (size_t)slice * wg_size(L);
+#pragma unroll
+  for (int j = 0; j < C::NTW; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = mg * 16 + g + (r >= 2 ? 8 : 0), q = (ng * C::NTW + j) * 8 + 2 * t + (r & 1);
+      if (q < NC) dst[(size_t)m * N + chunk * NC + q] = acc[j][r];
+    }
+  if (ng == 0 && chunk == 0) {
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      bs0 += __shfl_xor_sync(0xffffffffu, bs0, o);
+      bs1 += __shfl_xor_sync(0xffffffffu, bs1, o);
+    }
+    if (t == 0) {
+      dst[(size_t)c.co * N + mg * 16 + g] = bs0;
+      dst[(size_t)c.co * N + mg * 16 + g + 8] = bs1;
+    }
+  }
+}
+
+struct WgArgs {
+  const bf16 *in[4];
+  const float *g[4];
+};
+__global__ void __launch_bounds__(kTrThreads, 1) k_conv_wgrad(WgArgs A, WgPlan plan, int batch,
+                                                              bool words, float *__restrict__ part) {
+  const int b = blockIdx.x;
+  if (b < plan.first[1])
+    conv_wgrad<0>(A.in[0], A.g[0], batch, b, plan.slices[0], 0, words, part + plan.part[0]);
+  else if (b < plan.first[2])
+    conv_wgrad<1>(A.in[1], A.g[1], batch, b - plan.first[1], plan.slices[1], 0, true, part + plan.part[1]);
+  else if (b < plan.first[3])
+    conv_wgrad<2>(A.in[2], A.g[2], batch, b - plan.first[2], plan.slices[2], 0, true, part + plan.part[2]);
+  else
+    conv_wgrad<3>(A.in[3], A.g[3], batch, (b - plan.first[3]) / 4, plan.slices[3],
+                  (b - plan.first[3]) % 4, true, part + plan.part[3]);
+}
+
+// The conv weight and bias gradients from their slices (in slice order; a
+// layer's sums lie in parameter order), and the batch's mean loss (the last
+// block; a fixed tree).
+__global__ void __launch_bounds__(256) k_wgrad_reduce(WgPlan plan, const float *__restrict__ part,
+                                                      float *__restrict__ grad,
+                                                      float *__restrict__ loss, int batch,
+                                                      float *__restrict__ loss_out) {
+  if (blockIdx.x + 1 == gridDim.x) {
+    __shared__ float s[256];
+    float a = 0.f;
+    for (int b = threadIdx.x; b < batch; b += 256) a += loss[b];
+    s[threadIdx.x] = a;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      const float mean = s[0] / (float)batch;
+      loss[batch] = mean;
+      if (loss_out) *loss_out = mean;
+    }
+    return;
+  }
+  const long i = (long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= kOffF1) return;
+  const int l = i < kOffW1 ? 0 : i < kOffW2 ? 1 : i < kOffW3 ? 2 : 3;
+  const long off = l == 0 ? kOffW0 : l == 1 ? kOffW1 : l == 2 ? kOffW2 : kOffW3;
+  const int size = l == 0 ? wg_size(0) : l == 1 ? wg_size(1) : l == 2 ? wg_size(2) : wg_size(3);
+  const float *p = part + plan.part[l] + (i - off);
+  const int n = plan.slices[l];
+  float acc = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < n; ++s) acc += __ldg(p + (size_t)s * size);
+  grad[i] = acc;
+}
