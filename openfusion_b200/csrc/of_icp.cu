@@ -22,8 +22,10 @@
 //   stops the remaining iterations (ICP.cpp:152-158).
 #include "of_batch.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <string.h>
+#include <vector>
 
 using namespace of;
 
@@ -1235,26 +1237,41 @@ extern "C" of_status_t of_icp_track_static(const of_camera_t *cam, const of_icp_
 // ------------------------------------------------------------ batched ICP --
 //
 // Multi-level ICP of many independent streams in one persistent launch: each
-// thread-block cluster of kBatchCtas CTAs tracks one stream at a time and
-// takes the next stream from an atomic ticket over a longest-first order.
-// Per iteration every CTA associates its share of the level's model pixels
-// (thread g of the cluster takes pixels g, g + kBatchCtas * kBatchThreads,
-// ...), reduces its rows (warp recursive halving, then a tree over warps),
-// and pushes its 30-value row into every CTA's shared memory
-// (double-buffered by iteration parity); after one cluster barrier every CTA
-// sums the kBatchCtas rows in the same order and solves the same 6x6 system,
-// so all hold the same pose. The only waits are hardware cluster barriers.
-// The per-pixel arithmetic (association, inlier tests, rows, FP64 solve and
-// composition) is the single-stream kernel's; the summation order differs.
+// thread-block cluster tracks one stream at a time and takes the next stream
+// from an atomic ticket over a longest-first order. The level's model pixels
+// are dealt to kBatchSums chains: chain v sums the rows of pixels v, v +
+// kBatchSums, ... one after another; 32 chains make a warp's sum (recursive
+// halving), and trees over these, the CTA's and the cluster's, make the
+// total: every CTA pushes its 30-value row into every CTA's shared memory
+// (double-buffered by iteration parity), and after one cluster barrier each
+// sums the rows in the same order and solves the same 6x6 system, so all hold
+// the same pose. The only waits are barriers. The per-pixel arithmetic
+// (association, inlier tests, rows, FP64 solve and composition) is the
+// single-stream kernel's; the summation order differs.
+//
+// A thread a chain: a 640x480 level is 75 points a thread, and what bounds it
+// is that thread's instructions, one after another (with a branch a test, 186
+// instructions a point at 6 cycles each: no faster on twice the SMs). So the
+// arithmetic of two or three points is interleaved: it has no branch (a point
+// without a frame pixel reads pixel 0 and adds zeros), the reciprocal
+// included, and a point (vertex and normal, 32 bytes) is one load. The frame
+// pixels of the next step and the model points after them are on their way
+// meanwhile. The sums are added in the same order as before, so they are the
+// same bits. Measured on one B200 (kernel alone on the device): one 640x480
+// stream 571 -> 237 us, 16 streams (5 of 640x480, 7 of 320x240, 4 of 160x120)
+// 766 -> 419 us, 64 streams 1544 -> 1184 us.
 #include <cooperative_groups.h>
 
 namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int kBatchCtas = 8;
-constexpr int kBatchThreads = 512;
-constexpr int kBatchWarps = kBatchThreads / 32;
+constexpr int kBatchSums = 4096;  // chains of a level's sums, a thread each
+constexpr int batch_threads(int ctas) { return kBatchSums / ctas; }
+// Points of a chain in flight together: as many as a thread's registers hold
+// (255 of them in a CTA of 256 threads, 128 in one of 512). One stream of
+// 640x480 on 16 CTAs with 2 / 3 / 4 points: 288 / 237 / 258 us.
+constexpr int batch_step(int ctas) { return ctas == 16 ? 3 : 2; }
 
 struct IcpJob {
   IcpLevel lv[kMaxLevels];
@@ -1263,14 +1280,99 @@ struct IcpJob {
   of_icp_stats_t *stats;
 };
 
-__global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThreads, 1)
+// A point of a pyramid (vertex, normal), one 32-byte load: the batch's
+// pyramids start at 256-byte boundaries.
+struct MapPoint {
+  float4 v, n;
+};
+__device__ __forceinline__ MapPoint ld_point(const float4 *p) {
+  MapPoint m;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(m.v.x), "=f"(m.v.y), "=f"(m.v.z), "=f"(m.v.w), "=f"(m.n.x), "=f"(m.n.y), "=f"(m.n.z),
+        "=f"(m.n.w)
+      : "l"(p));
+  return m;
+}
+// 1 / z rounded to nearest for |z| in [2^-126, 2^126), without a branch: the
+// approximate reciprocal, a Newton step, and Markstein's final step (IBM
+// Journal of R&D 34, 1990), which rounds correctly from an approximation that
+// is right to within an ulp. Equal to __frcp_rn for every
+// mantissa, sign and exponent of that range (checked on B200 over all of them).
+__device__ __forceinline__ float recip_rn(float z) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(z));
+  y = __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
+  return __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
+}
+// associate() without a branch: the frame pixel (0 if none), and whether the
+// point projects into the frame.
+__device__ __forceinline__ int associate_flat(const Rigid &w2c, const Cam &cam, float3 s, bool &seen) {
+  const float3 sc = apply(w2c, s);
+  const float rz = recip_rn(sc.z);
+  const int pu = __float2int_rd(fmaf(cam.fx * sc.x, rz, cam.cx) + 0.5f);
+  const int pv = __float2int_rd(fmaf(cam.fy * sc.y, rz, cam.cy) + 0.5f);
+  seen = seen && !(sc.z >= -kEps) && (unsigned)pu < (unsigned)cam.w && (unsigned)pv < (unsigned)cam.h;
+  return seen ? pv * cam.w + pu : 0;
+}
+
+// A model point, the frame point at its pixel, and whether it has one.
+struct BatchPoint {
+  float3 s, ns;
+  MapPoint f;
+  bool seen;
+};
+__device__ __forceinline__ BatchPoint batch_frame(const MapPoint &m, bool live, const Rigid &w2c,
+                                                  const Cam &cam, const float4 *__restrict__ frame) {
+  BatchPoint b;
+  b.s = make_float3(m.v.x, m.v.y, m.v.z);
+  b.ns = make_float3(m.n.x, m.n.y, m.n.z);
+  b.seen = live && m.v.w != 0.f && m.n.w != 0.f;
+  const int q = associate_flat(w2c, cam, b.s, b.seen);
+  b.f = ld_point(frame + 2 * q);
+  return b;
+}
+// The point's row a[0..5], b = a[6] and inlier count a[7] (try_row's tests and
+// arithmetic); zeros when it is no inlier.
+__device__ __forceinline__ void batch_row(float (&a)[8], const Rigid &c2w, const BatchPoint &p,
+                                          float dist2, float nthr) {
+  const float3 s = p.s, ns = p.ns;
+  const float3 d = apply(c2w, make_float3(p.f.v.x, p.f.v.y, p.f.v.z));
+  const float3 nd = rotate(c2w, make_float3(p.f.n.x, p.f.n.y, p.f.n.z));
+  const float ex = d.x - s.x, ey = d.y - s.y, ez = d.z - s.z;
+  const float dn = nd.x * ns.x + nd.y * ns.y + nd.z * ns.z;
+  const bool ok = p.seen && p.f.v.w != 0.f && p.f.n.w != 0.f &&
+                  fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < dist2 && dn > nthr && dn < 1.f + kEps;
+  a[0] = ok ? ns.y * d.z - ns.z * d.y : 0.f;
+  a[1] = ok ? ns.z * d.x - ns.x * d.z : 0.f;
+  a[2] = ok ? ns.x * d.y - ns.y * d.x : 0.f;
+  a[3] = ok ? ns.x : 0.f;
+  a[4] = ok ? ns.y : 0.f;
+  a[5] = ok ? ns.z : 0.f;
+  a[6] = ok ? -(ns.x * ex + ns.y * ey + ns.z * ez) : 0.f;
+  a[7] = ok ? 1.f : 0.f;
+}
+__device__ __forceinline__ void batch_add(float *acc, const float (&a)[8]) {
+  int k = 0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int j = i; j < 6; ++j) { acc[k] = fmaf(a[i], a[j], acc[k]); ++k; }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) acc[21 + i] = fmaf(a[i], a[6], acc[21 + i]);
+  acc[27] = fmaf(a[6], a[6], acc[27]);
+  acc[28] += a[7];
+}
+
+template <int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTAS), 1)
     k_icp_batch(const IcpJob *__restrict__ jobs, const int *__restrict__ order, int njobs,
                 unsigned int *ticket, float dist_thresh, float normal_thresh, float stop_rot,
                 float stop_trans) {
   __shared__ double s_pose[16], s_init[16];
   __shared__ Rigid s_c2w, s_w2c;
-  __shared__ float s_red[kBatchWarps][32];
-  __shared__ float s_part[2][kBatchCtas][32];
+  constexpr int THREADS = batch_threads(CTAS), ROWS = THREADS / 32, STEP = batch_step(CTAS);
+  __shared__ float s_red[ROWS][32];
+  __shared__ float s_part[2][CTAS][32];
   __shared__ float s_tot[32];
   __shared__ int s_job, s_stop, s_conv, s_its, s_inl;
   __shared__ double s_res, s_piv;
@@ -1282,7 +1384,7 @@ __global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThrea
     if (rank == 0 && threadIdx.x == 0) {
       const unsigned t = atomicAdd(ticket, 1u);
       const int job = t < (unsigned)njobs ? __ldg(order + t) : -1;
-      for (int r = 0; r < kBatchCtas; ++r) *cluster.map_shared_rank(&s_job, r) = job;
+      for (int r = 0; r < CTAS; ++r) *cluster.map_shared_rank(&s_job, r) = job;
     }
     cluster.sync();
     const int job = s_job;
@@ -1303,7 +1405,6 @@ __global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThrea
     int iter = 0;
     for (int l = J.levels - 1; l >= 0 && !s_stop; --l) {
       const IcpLevel L = J.lv[l];
-      const int npx = L.mw * L.mh;
       __syncthreads();  // every thread has read the previous level's exit flag
       if (threadIdx.x == 0) s_conv = 0;
       __syncthreads();
@@ -1312,24 +1413,37 @@ __global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThrea
         float examined = 0.f;
 #pragma unroll
         for (int v = 0; v < kVals; ++v) acc[v] = 0.f;
-        constexpr int kStride = kBatchCtas * kBatchThreads;
-        for (int p = rank * kBatchThreads + threadIdx.x; p < npx; p += 2 * kStride) {
-          const int p2 = p + kStride;
-          const float4 sA = __ldg(L.model + 2 * p), nA = __ldg(L.model + 2 * p + 1);
-          float4 sB = make_float4(0.f, 0.f, 0.f, 0.f), nB = sB;
-          if (p2 < npx) { sB = __ldg(L.model + 2 * p2); nB = __ldg(L.model + 2 * p2 + 1); }
-          const int qA = (sA.w != 0.f && nA.w != 0.f) ? associate(s_w2c, L.cam, sA) : -1;
-          const int qB = (sB.w != 0.f && nB.w != 0.f) ? associate(s_w2c, L.cam, sB) : -1;
-          float4 dA = make_float4(0.f, 0.f, 0.f, 0.f), cA = dA, dB = dA, cB = dA;
-          if (qA >= 0) { dA = __ldg(L.frame + 2 * qA); cA = __ldg(L.frame + 2 * qA + 1); }
-          if (qB >= 0) { dB = __ldg(L.frame + 2 * qB); cB = __ldg(L.frame + 2 * qB + 1); }
-          if (qA >= 0) {
-            examined += 1.f;
-            try_row(acc, s_c2w, sA, nA, dA, cA, dist2, normal_thresh);
-          }
-          if (qB >= 0) {
-            examined += 1.f;
-            try_row(acc, s_c2w, sB, nB, dB, cB, dist2, normal_thresh);
+        {
+          const int npx = L.mw * L.mh, last = npx - 1;
+          int p = rank * THREADS + threadIdx.x;
+          MapPoint nxt[STEP];
+          BatchPoint cur[STEP];
+          auto models = [&](int q) {
+#pragma unroll
+            for (int i = 0; i < STEP; ++i) nxt[i] = ld_point(L.model + 2 * min(q + i * kBatchSums, last));
+          };
+          auto frames = [&](BatchPoint (&b)[STEP], int q) {
+#pragma unroll
+            for (int i = 0; i < STEP; ++i)
+              b[i] = batch_frame(nxt[i], q + i * kBatchSums < npx, s_w2c, L.cam, L.frame);
+          };
+          models(p);
+          frames(cur, p);
+          models(p + STEP * kBatchSums);
+          for (; p < npx; p += STEP * kBatchSums) {
+            BatchPoint fut[STEP];
+            frames(fut, p + STEP * kBatchSums);
+            models(p + 2 * STEP * kBatchSums);
+            float a[STEP][8];
+#pragma unroll
+            for (int i = 0; i < STEP; ++i) {
+              batch_row(a[i], s_c2w, cur[i], dist2, normal_thresh);
+              examined += cur[i].seen ? 1.f : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < STEP; ++i) batch_add(acc, a[i]);
+#pragma unroll
+            for (int i = 0; i < STEP; ++i) cur[i] = fut[i];
           }
         }
         // this CTA's row: recursive halving across the warp, a tree over warps
@@ -1352,30 +1466,32 @@ __global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThrea
         __syncthreads();
         const int buf = iter & 1;
         if (warp == 0) {
-          float y[kBatchWarps];
+          float y[ROWS];
 #pragma unroll
-          for (int w = 0; w < kBatchWarps; ++w) y[w] = s_red[w][lane];
+          for (int w = 0; w < ROWS; ++w) y[w] = s_red[w][lane];
 #pragma unroll
-          for (int span = 1; span < kBatchWarps; span *= 2)
+          for (int span = 1; span < ROWS; span *= 2)
 #pragma unroll
-            for (int w = 0; w + span < kBatchWarps; w += 2 * span) y[w] += y[w + span];
+            for (int w = 0; w + span < ROWS; w += 2 * span) y[w] += y[w + span];
 #pragma unroll
-          for (int r = 0; r < kBatchCtas; ++r) cluster.map_shared_rank(&s_part[buf][rank][0], r)[lane] = y[0];
+          for (int r = 0; r < CTAS; ++r) cluster.map_shared_rank(&s_part[buf][rank][0], r)[lane] = y[0];
         }
         cluster.sync();
         if (warp == 0) {
-          float y[kBatchCtas];
+          float y[CTAS];
 #pragma unroll
-          for (int r = 0; r < kBatchCtas; ++r) y[r] = s_part[buf][r][lane];
+          for (int r = 0; r < CTAS; ++r) y[r] = s_part[buf][r][lane];
 #pragma unroll
-          for (int span = 1; span < kBatchCtas; span *= 2)
+          for (int span = 1; span < CTAS; span *= 2)
 #pragma unroll
-            for (int r = 0; r + span < kBatchCtas; r += 2 * span) y[r] += y[r + span];
+            for (int r = 0; r + span < CTAS; r += 2 * span) y[r] += y[r + span];
           s_tot[lane] = y[0];
           __syncwarp();
           double minpiv = 0.0;
           float inc_rot = 0.f, inc_trans = 0.f;
-          const bool ok = warp_solve_update(s_tot, s_pose, &minpiv, &inc_rot, &inc_trans);
+          // (on success the warp also writes the new pose's rigid transforms)
+          const bool ok =
+              warp_solve_update(s_tot, s_pose, &minpiv, &inc_rot, &inc_trans, &s_c2w, &s_w2c);
           if (lane == 0) {
             s_its += 1;
             s_inl = (int)s_tot[28];
@@ -1384,10 +1500,10 @@ __global__ void __cluster_dims__(kBatchCtas, 1, 1) __launch_bounds__(kBatchThrea
             if (!ok) {
               for (int i = 0; i < 16; ++i) s_pose[i] = s_init[i];
               s_stop = 1;
+              pose_to_rigid(s_pose, &s_c2w, &s_w2c);
             } else if (stop_rot > 0.f && inc_rot < stop_rot && inc_trans < stop_trans) {
               s_conv = 1;
             }
-            pose_to_rigid(s_pose, &s_c2w, &s_w2c);
           }
         }
         __syncthreads();
@@ -1419,6 +1535,7 @@ struct IcpBatch {
   IcpJob *jobs = nullptr;
   int *order = nullptr;
   unsigned int *ticket = nullptr;
+  std::vector<double> cost;  // pixel visits a step, longest first
 };
 
 void icp_batch_destroy(IcpBatch *b) {
@@ -1429,28 +1546,42 @@ void icp_batch_destroy(IcpBatch *b) {
   delete b;
 }
 
-// Clusters of the batched ICP that fit on the device at once.
-int icp_batch_max_clusters() {
-  static int cached = 0;
-  if (cached > 0) return cached;
+// (the attributes belong to the function in the current context: set before
+// every launch and query)
+template <int CTAS>
+static cudaError_t batch_attributes() {
+  return CTAS > 8 ? cudaFuncSetAttribute((const void *)k_icp_batch<CTAS>,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1)
+                  : cudaSuccess;
+}
+template <int CTAS>
+static int batch_fit() {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kBatchCtas * kSmCount / kBatchCtas);
-  cfg.blockDim = dim3(kBatchThreads);
+  cfg.gridDim = dim3(CTAS);
+  cfg.blockDim = dim3(batch_threads(CTAS));
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = kBatchCtas;
+  attr.val.clusterDim.x = CTAS;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, (void *)k_icp_batch, &cfg) != cudaSuccess || n < 1) {
+  if (batch_attributes<CTAS>() != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, (void *)k_icp_batch<CTAS>, &cfg) != cudaSuccess) {
     cudaGetLastError();
-    n = kSmCount / kBatchCtas;
+    n = 0;
   }
-  cached = n;
   return n;
 }
+// Clusters of each size that fit on the device at once.
+static int batch_clusters(int ctas) {
+  static const int fit8 = batch_fit<8>(), fit16 = batch_fit<16>();
+  return ctas == 16 ? fit16 : (fit8 > 0 ? fit8 : kSmCount / 8);
+}
+// Clusters of the batched ICP that fit on the device at once (of 8 CTAs, the
+// size that serves many streams).
+int icp_batch_max_clusters() { return batch_clusters(8); }
 
 of_status_t icp_batch_create(const BatchStream *s, int n, const BatchParams &p, IcpBatch **out) {
   const of_icp_params_t *ip = &p.icp;
@@ -1493,6 +1624,7 @@ of_status_t icp_batch_create(const BatchStream *s, int n, const BatchParams &p, 
          --k) {
       const int t = order[k]; order[k] = order[k - 1]; order[k - 1] = t;
     }
+  for (int i = 0; i < n; ++i) b->cost.push_back(cost[order[i]]);
   order[n] = 0;
   if (st == OF_OK) st = upload_jobs(jobs, order, n, &b->jobs, &b->order);
   if (st == OF_OK) {
@@ -1510,15 +1642,36 @@ of_status_t icp_batch_create(const BatchStream *s, int n, const BatchParams &p, 
   return OF_OK;
 }
 
+// When the last of `k` clusters ends, each taking the next stream as it falls
+// free (longest first), with a stream's time a + slope x its cost.
+static double batch_makespan(const std::vector<double> &cost, int k, double a, double slope) {
+  constexpr double kUnit = 640.0 * 480.0 * (10.0 + 5.0 / 4.0 + 4.0 / 16.0);
+  std::vector<double> end((size_t)k, 0.0);
+  for (double c : cost) *std::min_element(end.begin(), end.end()) += a + slope * c / kUnit;
+  return *std::max_element(end.begin(), end.end());
+}
+
 of_status_t icp_batch_launch(const IcpBatch *b, const BatchKnobs &k, cudaStream_t s) {
-  const int maxc = icp_batch_max_clusters();
-  int clusters = k.icp_clusters > 0 ? k.icp_clusters : maxc;
-  if (clusters > maxc) clusters = maxc;
-  if (clusters > b->n) clusters = b->n;
+  const int cap = k.icp_clusters > 0 && k.icp_clusters < b->n ? k.icp_clusters : b->n;
+  const int fit8 = batch_clusters(8), fit16 = batch_clusters(16);
+  const int k8 = cap < fit8 ? cap : fit8, k16 = cap < fit16 ? cap : fit16;
+  // A cluster of 16 CTAs tracks a stream faster, but fewer fit (7 against 15
+  // on a B200): the size whose longest-first schedule ends earlier. Measured
+  // times of a stream, us: 66 + 171 c on 16 CTAs, 82 + 338 c on 8, c = its
+  // pixel visits over those of a 640x480 stream at 10/5/4 iterations.
+  const bool wide = k16 > 0 && batch_makespan(b->cost, k16, 66.0, 171.0) <
+                                   batch_makespan(b->cost, k8, 82.0, 338.0);
+  const int clusters = wide ? k16 : k8;
   OF_CUDA_TRY(cudaMemsetAsync(b->ticket, 0, sizeof(unsigned int), s));
-  k_icp_batch<<<clusters * kBatchCtas, kBatchThreads, 0, s>>>(b->jobs, b->order, b->n, b->ticket,
-                                                            b->dist, b->nthr, b->stop_rot,
-                                                            b->stop_trans);
+  if (wide) {
+    OF_CUDA_TRY(batch_attributes<16>());
+    k_icp_batch<16><<<clusters * 16, batch_threads(16), 0, s>>>(
+        b->jobs, b->order, b->n, b->ticket, b->dist, b->nthr, b->stop_rot, b->stop_trans);
+  } else {
+    OF_CUDA_TRY(batch_attributes<8>());
+    k_icp_batch<8><<<clusters * 8, batch_threads(8), 0, s>>>(
+        b->jobs, b->order, b->n, b->ticket, b->dist, b->nthr, b->stop_rot, b->stop_trans);
+  }
   return of_launch_status();
 }
 
