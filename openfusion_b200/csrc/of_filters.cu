@@ -11,10 +11,12 @@
 // outside the image (the reference leaves them unwritten, :191-193) or whose
 // bilinear taps include a null pixel (it would blend a null into the depth),
 // and treats the last row like the last column (the reference compares the
-// column with the height there, :207). Chained filters run back to back on
-// one stream through a ping-pong buffer (the reference synchronises the
-// device and copies the result back after every filter, :131-151).
+// column with the height there, :207). A chain of filters is one launch (the
+// reference synchronises the device and copies the result back after every
+// filter, :131-151).
 #include "of_common.cuh"
+
+#include <utility>
 
 using namespace of;
 
@@ -22,129 +24,222 @@ bool of_camera_valid(const of_camera_t *c);
 
 namespace {
 
-constexpr int kFx = 32, kFy = 8;
-
-// Median of the window's non-null pixels by rank selection in registers:
-// keys of null or outside pixels are 0x10000 (above every depth), so the
-// valid values' ranks are their ranks among the valid ones.
-__global__ void __launch_bounds__(kFx * kFy) k_median5(const uint16_t *__restrict__ in,
-                                                       uint16_t *__restrict__ out, int w, int h,
-                                                       uint32_t nullv) {
-  const int x = blockIdx.x * kFx + threadIdx.x, y = blockIdx.y * kFy + threadIdx.y;
-  if (x >= w || y >= h) return;
-  uint32_t key[25];
-  int n = 0, win = 0;
-#pragma unroll
-  for (int j = 0; j < 5; ++j)
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const int xx = x + i - 2, yy = y + j - 2;
-      uint32_t k = 0x10000u;
-      if ((unsigned)xx < (unsigned)w && (unsigned)yy < (unsigned)h) {
-        ++win;
-        const uint32_t d = __ldg(in + (size_t)yy * w + xx);
-        if (d != nullv) { k = d; ++n; }
-      }
-      key[j * 5 + i] = k;
-    }
-  uint32_t r = nullv;
-  if (n > win / 2) {
-    // order statistics k0 = (n - 1) / 2 and k1 = n / 2 (equal for odd n)
-    const int k0 = (n - 1) >> 1, k1 = n >> 1;
-    uint32_t v0 = 0, v1 = 0;
-#pragma unroll
-    for (int a = 0; a < 25; ++a) {
-      int less = 0, leq = 0;
-#pragma unroll
-      for (int b = 0; b < 25; ++b) {
-        less += key[b] < key[a];
-        leq += key[b] <= key[a];
-      }
-      if (key[a] < 0x10000u) {
-        if (less <= k0 && k0 < leq) v0 = key[a];
-        if (less <= k1 && k1 < leq) v1 = key[a];
-      }
-    }
-    r = (n & 1) ? v1 : (v0 + v1) >> 1;
-  }
-  out[(size_t)y * w + x] = (uint16_t)r;
-}
-
-__global__ void __launch_bounds__(kFx * kFy) k_average(const uint16_t *__restrict__ in,
-                                                       uint16_t *__restrict__ out, int w, int h,
-                                                       uint32_t nullv, float thr) {
-  const int x = blockIdx.x * kFx + threadIdx.x, y = blockIdx.y * kFy + threadIdx.y;
-  if (x >= w || y >= h) return;
-  float s = 0.f;
-  int n = 0;
-#pragma unroll
-  for (int j = -1; j <= 1; ++j)
-#pragma unroll
-    for (int i = -1; i <= 1; ++i) {
-      const int xx = x + i, yy = y + j;
-      if ((i == 0 && j == 0) || (unsigned)xx >= (unsigned)w || (unsigned)yy >= (unsigned)h) continue;
-      s += (float)__ldg(in + (size_t)yy * w + xx);
-      ++n;
-    }
-  const float avg = s / (float)n;
-  const float v = (float)__ldg(in + (size_t)y * w + x);
-  out[(size_t)y * w + x] = fabsf(avg - v) > thr ? (uint16_t)nullv : (uint16_t)avg;
-}
-
-__global__ void __launch_bounds__(kFx * kFy) k_gradient(const uint16_t *__restrict__ in,
-                                                        uint16_t *__restrict__ out, int w, int h,
-                                                        double thr36) {
-  const int x = blockIdx.x * kFx + threadIdx.x, y = blockIdx.y * kFy + threadIdx.y;
-  if (x >= w || y >= h) return;
-  const int xm = max(x - 1, 0), xp = min(x + 1, w - 1), ym = max(y - 1, 0), yp = min(y + 1, h - 1);
-  const int cols[3] = {xm, x, xp}, rows[3] = {ym, y, yp};
-  long long gx = 0, gy = 0;
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-    gx += (long long)__ldg(in + (size_t)rows[j] * w + xp) - __ldg(in + (size_t)rows[j] * w + xm);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-    gy += (long long)__ldg(in + (size_t)yp * w + cols[i]) - __ldg(in + (size_t)ym * w + cols[i]);
-  // (gx / 6)^2 + (gy / 6)^2 > thr^2, exactly: gx^2 + gy^2 > 36 thr^2
-  const double g2 = (double)(gx * gx + gy * gy);
-  out[(size_t)y * w + x] = g2 > thr36 ? (uint16_t)0 : __ldg(in + (size_t)y * w + x);
-}
+// One launch runs a whole chain: a block holds a tile of the image with the
+// chain's halo (2 pixels for the median, 1 for every other step) in shared
+// memory and applies the steps there, each on a region smaller by its radius,
+// so an image is read and written once however long the chain. The halo is
+// filtered again by each neighbour (1.5 x the tile for median, gradient and
+// two averages), which costs less than a launch and a pass over memory a step.
+// Measured at 640x480, median + gradient + two averages: a kernel a step, the
+// median by ranking each of 25 values against the others, 65 us; this form
+// 18 us (kernel 14).
+// (tiles of 64 x 17: a 640x480 image is 290 blocks, one wave of two an SM)
+constexpr int kTx = 64, kTy = 17, kChainThreads = 512;
 
 struct Brown {
   float fx, fy, cx, cy, k1, k2, p1, p2;
 };
+struct Chain {
+  int w, h;
+  int steps, halo;
+  uint32_t kinds;                 // OF_DEPTH_FILTER_* in shared memory, in order, 4 bits each
+  bool undistort;                 // while the tile is loaded
+  uint32_t nullv;
+  float avg_thr;
+  double grad36;  // 36 x the gradient threshold squared
+  Brown B;
+};
 
-__global__ void __launch_bounds__(kFx * kFy) k_undistort(const uint16_t *__restrict__ in,
-                                                         uint16_t *__restrict__ out, int w, int h,
-                                                         Brown B, uint32_t nullv) {
-  const int x = blockIdx.x * kFx + threadIdx.x, y = blockIdx.y * kFy + threadIdx.y;
-  if (x >= w || y >= h) return;
+__device__ __forceinline__ uint32_t undistorted(const uint16_t *__restrict__ in, int w, int h,
+                                                const Brown &B, uint32_t nullv, int x, int y) {
   const float xn = ((float)x - B.cx) / B.fx, yn = ((float)y - B.cy) / B.fy;
   const float r2 = xn * xn + yn * yn, rad = 1.f + B.k1 * r2 + B.k2 * r2 * r2;
   const float xd = xn * rad + 2.f * B.p1 * xn * yn + B.p2 * (r2 + 2.f * xn * xn);
   const float yd = yn * rad + B.p1 * (r2 + 2.f * yn * yn) + 2.f * B.p2 * xn * yn;
   const float u = B.fx * xd + B.cx, v = B.fy * yd + B.cy;
   const float u0f = floorf(u), v0f = floorf(v);
-  const size_t o = (size_t)y * w + x;
-  if (!(u0f >= 0.f && u0f <= (float)(w - 1) && v0f >= 0.f && v0f <= (float)(h - 1))) {
-    out[o] = (uint16_t)nullv;
-    return;
-  }
+  if (!(u0f >= 0.f && u0f <= (float)(w - 1) && v0f >= 0.f && v0f <= (float)(h - 1))) return nullv;
   const int u0 = (int)u0f, v0 = (int)v0f;
   const int u1 = u0 + 1 < w ? u0 + 1 : u0, v1 = v0 + 1 < h ? v0 + 1 : v0;
   const uint32_t a = __ldg(in + (size_t)v0 * w + u0), b = __ldg(in + (size_t)v0 * w + u1);
   const uint32_t c = __ldg(in + (size_t)v1 * w + u0), d = __ldg(in + (size_t)v1 * w + u1);
-  if (a == nullv || b == nullv || c == nullv || d == nullv) {
-    out[o] = (uint16_t)nullv;
-    return;
-  }
+  if (a == nullv || b == nullv || c == nullv || d == nullv) return nullv;
   const float fu = u - u0f, fv = v - v0f;
   const uint32_t f1 = u1 == u0 ? a : (uint32_t)((1.f - fu) * (float)a + fu * (float)b);
   const uint32_t f2 = v1 == v0 ? f1 : (u1 == u0 ? c : (uint32_t)((1.f - fu) * (float)c + fu * (float)d));
-  out[o] = (uint16_t)(uint32_t)((1.f - fv) * (float)f1 + fv * (float)f2);
+  return (uint16_t)(uint32_t)((1.f - fv) * (float)f1 + fv * (float)f2);
 }
 
-dim3 grid_of(int w, int h) { return dim3((w + kFx - 1) / kFx, (h + kFy - 1) / kFy); }
+// Batcher's merge exchange for 25 keys (Knuth, TAOCP 5.2.2, algorithm M) as a
+// list of exchanges.
+struct MergePair {
+  int i, j;
+};
+constexpr int kMergePairs = 138;
+struct MergeList {
+  MergePair x[kMergePairs];
+  int n;
+};
+constexpr MergeList merge_list() {
+  MergeList L = {};
+  for (int p = 16; p > 0; p >>= 1) {
+    for (int i = 0; i < 25 - p; ++i)
+      if ((i & p) == 0) L.x[L.n++] = {i, i + p};
+    for (int q = 16; q != p; q >>= 1)
+      for (int i = 0; i < 25 - (q - p); ++i)
+        if ((i & p) == p) L.x[L.n++] = {i, i + q - p};
+  }
+  return L;
+}
+static_assert(merge_list().n == kMergePairs, "exchanges");
+template <int N>
+__device__ __forceinline__ void merge_exchange(uint32_t (&k)[25]) {
+  constexpr MergePair e = merge_list().x[N];
+  const uint32_t lo = __vminu2(k[e.i], k[e.j]);
+  k[e.j] = __vmaxu2(k[e.i], k[e.j]);
+  k[e.i] = lo;
+}
+template <size_t... N>
+__device__ __forceinline__ void run_merge(uint32_t (&k)[25], std::index_sequence<N...>) {
+  (merge_exchange<(int)N>(k), ...);
+}
+
+// Medians of the 5x5 windows of two neighbouring pixels, x (low half) and x +
+// 1 (high half), `s` the tile at (x - 2, y - 2) (an even column), rows `pitch`
+// apart; nulls and pixels outside the image hold `nullv`. Of a window's m
+// nulls, floor(m / 2) become 0 and the others 0xffff, so that the middle of all
+// 25 keys is the middle of the valid ones: position 12, and with it position
+// 11 when their number is even. The exchanges work on 16-bit pairs, two pixels
+// an instruction; the compiler drops those that reach neither position.
+__device__ __forceinline__ void median_pair(const uint16_t *s, int pitch, uint32_t nullv,
+                                            uint32_t &m11, uint32_t &m12, uint32_t &nulls) {
+  const uint32_t null2 = nullv | nullv << 16;
+  uint32_t k[25];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(s + j * pitch);
+    const uint32_t a = row[0], b = row[1], c = row[2];
+    k[5 * j] = a;
+    k[5 * j + 1] = __byte_perm(a, b, 0x5432);
+    k[5 * j + 2] = b;
+    k[5 * j + 3] = __byte_perm(b, c, 0x5432);
+    k[5 * j + 4] = c;
+  }
+  uint32_t pad = 0xffffffffu;  // the next null's key, per half
+  nulls = 0;
+#pragma unroll
+  for (int i = 0; i < 25; ++i) {
+    const uint32_t one = __vminu2(k[i] ^ null2, 0x00010001u) ^ 0x00010001u;  // 1 per null half
+    const uint32_t mask = one * 0xffffu;
+    k[i] = (k[i] & ~mask) | (mask & pad);
+    pad ^= mask;
+    nulls += one;
+  }
+  run_merge(k, std::make_index_sequence<kMergePairs>());
+  m11 = k[11];
+  m12 = k[12];
+}
+
+__global__ void __launch_bounds__(kChainThreads) k_filter_chain(const uint16_t *__restrict__ in,
+                                                                uint16_t *__restrict__ out, Chain C) {
+  extern __shared__ __align__(8) uint16_t s_tile[];
+  const int H = C.halo, w = C.w, h = C.h;
+  const int RW = (kTx + 2 * H + 3) & ~1, RH = kTy + 2 * H;  // (an even pitch, a column to spare)
+  uint16_t *src = s_tile, *dst = s_tile + RW * RH;
+  const int gx0 = blockIdx.x * kTx - H, gy0 = blockIdx.y * kTy - H;
+  // the cells of a rows x cols region, dealt to the threads in a row: i / cols
+  // by a 22-bit reciprocal (exact for i < 2^13, cols < 2^9)
+  auto each = [](int rows, int cols, auto f) {
+    const unsigned inv = (1u << 22) / (unsigned)cols + 1u;
+    for (int i = threadIdx.x; i < rows * cols; i += kChainThreads) {
+      const int r = (int)(((unsigned)i * inv) >> 22);
+      f(r, i - r * cols);
+    }
+  };
+  each(RH, RW, [&](int ry, int rx) {
+    const int x = gx0 + rx, y = gy0 + ry;
+    uint32_t d = C.nullv;
+    if ((unsigned)x < (unsigned)w && (unsigned)y < (unsigned)h)
+      d = C.undistort ? undistorted(in, w, h, C.B, C.nullv, x, y) : __ldg(in + (size_t)y * w + x);
+    src[ry * RW + rx] = (uint16_t)d;
+  });
+  __syncthreads();
+  int m = H;  // the margin around the tile that `src` holds
+  for (int st = 0; st < C.steps; ++st) {
+    const int kind = (int)(C.kinds >> (4 * st)) & 15;
+    m -= kind == OF_DEPTH_FILTER_MEDIAN5 ? 2 : 1;
+    const int x0 = H - m, y0 = H - m, cols = kTx + 2 * m, rows = kTy + 2 * m;
+    if (kind == OF_DEPTH_FILTER_MEDIAN5) {
+      const int xe = x0 & ~1;
+      each(rows, (x0 + cols - xe + 1) / 2, [&](int r, int c) {
+        const int ry = y0 + r, rx = xe + 2 * c, y = gy0 + ry;
+        if ((unsigned)y >= (unsigned)h) return;
+        uint32_t a, b, nulls;
+        median_pair(src + (ry - 2) * RW + rx - 2, RW, C.nullv, a, b, nulls);
+        const int wy = min(y + 2, h - 1) - max(y - 2, 0) + 1;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int x = gx0 + rx + e;
+          if ((unsigned)x >= (unsigned)w) continue;
+          const int win = wy * (min(x + 2, w - 1) - max(x - 2, 0) + 1);
+          const int n = 25 - (int)((nulls >> (16 * e)) & 0xffffu);
+          const uint32_t v0 = (a >> (16 * e)) & 0xffffu, v1 = (b >> (16 * e)) & 0xffffu;
+          dst[ry * RW + rx + e] =
+              (uint16_t)(n > win / 2 ? ((n & 1) ? v1 : (v0 + v1) >> 1) : C.nullv);
+        }
+      });
+    } else {
+      // no pixel of the region on the image's edge, nor outside
+      const bool inner = gx0 + x0 > 0 && gx0 + x0 + cols < w && gy0 + y0 > 0 && gy0 + y0 + rows < h;
+      each(rows, cols, [&](int r, int cc) {
+        const int ry = y0 + r, rx = x0 + cc, x = gx0 + rx, y = gy0 + ry;
+        if ((unsigned)x >= (unsigned)w || (unsigned)y >= (unsigned)h) return;
+        const uint16_t *c = src + ry * RW + rx;
+        uint32_t v;
+        if (kind == OF_DEPTH_FILTER_GRADIENT) {
+          // (clamped neighbours)
+          const int xm = x > 0 ? -1 : 0, xp = x + 1 < w ? 1 : 0;
+          const int ym = y > 0 ? -RW : 0, yp = y + 1 < h ? RW : 0;
+          const int gx = ((int)c[ym + xp] - (int)c[ym + xm]) + ((int)c[xp] - (int)c[xm]) +
+                         ((int)c[yp + xp] - (int)c[yp + xm]);
+          const int gy = ((int)c[yp + xm] - (int)c[ym + xm]) + ((int)c[yp] - (int)c[ym]) +
+                         ((int)c[yp + xp] - (int)c[ym + xp]);
+          // (gx / 6)^2 + (gy / 6)^2 > thr^2, exactly: gx^2 + gy^2 > 36 thr^2
+          v = (double)((long long)gx * gx + (long long)gy * gy) > C.grad36 ? 0u : c[0];
+        } else if (inner) {
+          // (whole numbers below 2^24: exact in any order)
+          const int s = (int)c[-RW - 1] + c[-RW] + c[-RW + 1] + c[-1] + c[1] + c[RW - 1] + c[RW] + c[RW + 1];
+          const float avg = (float)s * 0.125f;
+          v = fabsf(avg - (float)c[0]) > C.avg_thr ? C.nullv : (uint32_t)s >> 3;
+        } else {
+          float s = 0.f;
+          int n = 0;
+#pragma unroll
+          for (int j = -1; j <= 1; ++j)
+#pragma unroll
+            for (int i = -1; i <= 1; ++i) {
+              if ((i == 0 && j == 0) || (unsigned)(x + i) >= (unsigned)w ||
+                  (unsigned)(y + j) >= (unsigned)h)
+                continue;
+              s += (float)c[j * RW + i];
+              ++n;
+            }
+          const float avg = s / (float)n;
+          v = fabsf(avg - (float)c[0]) > C.avg_thr ? C.nullv : (uint32_t)(uint16_t)avg;
+        }
+        dst[ry * RW + rx] = (uint16_t)v;
+      });
+    }
+    __syncthreads();
+    uint16_t *t = src;
+    src = dst;
+    dst = t;
+  }
+  each(kTy, kTx, [&](int r, int c) {
+    const int x = gx0 + H + c, y = gy0 + H + r;
+    if (x < w && y < h) out[(size_t)y * w + x] = src[(H + r) * RW + H + c];
+  });
+}
 
 bool filter_params_ok(const of_depth_filter_params_t *p) {
   return p && (p->steps & ~0xF) == 0 && p->null_value >= 0 && p->null_value <= 0xFFFF &&
@@ -152,30 +247,29 @@ bool filter_params_ok(const of_depth_filter_params_t *p) {
          p->gradient_threshold_mm >= 0.f;
 }
 
-// one filter step (kind = one OF_DEPTH_FILTER_* bit) from src to dst (distinct)
-of_status_t launch_step(int kind, const of_camera_t *cam, const of_depth_filter_params_t *p,
-                        const uint16_t *src, uint16_t *dst, cudaStream_t s) {
-  const int w = cam->width, h = cam->height;
-  const uint32_t nv = (uint32_t)p->null_value;
-  switch (kind) {
-    case OF_DEPTH_FILTER_UNDISTORT: {
-      Brown B{cam->fx, cam->fy, cam->cx, cam->cy, p->k1, p->k2, p->p1, p->p2};
-      k_undistort<<<grid_of(w, h), dim3(kFx, kFy), 0, s>>>(src, dst, w, h, B, nv);
-      break;
+// the steps of `kinds` (OF_DEPTH_FILTER_* bits, undistortion first) from src
+// to dst (distinct), one launch
+of_status_t launch_chain(const int *kinds, int count, const of_camera_t *cam,
+                         const of_depth_filter_params_t *p, const uint16_t *src, uint16_t *dst,
+                         cudaStream_t s) {
+  Chain C = {};
+  C.w = cam->width;
+  C.h = cam->height;
+  C.nullv = (uint32_t)p->null_value;
+  C.avg_thr = p->average_threshold_mm;
+  C.grad36 = 36.0 * (double)p->gradient_threshold_mm * p->gradient_threshold_mm;
+  C.B = {cam->fx, cam->fy, cam->cx, cam->cy, p->k1, p->k2, p->p1, p->p2};
+  for (int i = 0; i < count; ++i) {
+    if (kinds[i] == OF_DEPTH_FILTER_UNDISTORT) {
+      C.undistort = true;
+      continue;
     }
-    case OF_DEPTH_FILTER_MEDIAN5:
-      k_median5<<<grid_of(w, h), dim3(kFx, kFy), 0, s>>>(src, dst, w, h, nv);
-      break;
-    case OF_DEPTH_FILTER_GRADIENT:
-      k_gradient<<<grid_of(w, h), dim3(kFx, kFy), 0, s>>>(
-          src, dst, w, h, 36.0 * (double)p->gradient_threshold_mm * p->gradient_threshold_mm);
-      break;
-    case OF_DEPTH_FILTER_AVERAGE:
-      k_average<<<grid_of(w, h), dim3(kFx, kFy), 0, s>>>(src, dst, w, h, nv, p->average_threshold_mm);
-      break;
-    default:
-      return OF_ERR_INVALID_ARGUMENT;
+    C.kinds |= (uint32_t)kinds[i] << (4 * C.steps++);  // (at most 6: median, gradient, 4 averages)
+    C.halo += kinds[i] == OF_DEPTH_FILTER_MEDIAN5 ? 2 : 1;
   }
+  const int RW = (kTx + 2 * C.halo + 3) & ~1, RH = kTy + 2 * C.halo;
+  const dim3 grid((C.w + kTx - 1) / kTx, (C.h + kTy - 1) / kTy);
+  k_filter_chain<<<grid, kChainThreads, 2 * RW * RH * sizeof(uint16_t), s>>>(src, dst, C);
   return of_launch_status();
 }
 
@@ -188,7 +282,7 @@ extern "C" of_status_t of_depth_filter_step(const of_camera_t *cam, int32_t kind
       (kind != OF_DEPTH_FILTER_UNDISTORT && kind != OF_DEPTH_FILTER_MEDIAN5 &&
        kind != OF_DEPTH_FILTER_GRADIENT && kind != OF_DEPTH_FILTER_AVERAGE))
     return OF_ERR_INVALID_ARGUMENT;
-  return launch_step(kind, cam, p, d_in, d_out, (cudaStream_t)stream);
+  return launch_chain(&kind, 1, cam, p, d_in, d_out, (cudaStream_t)stream);
 }
 
 extern "C" of_status_t of_depth_filter(const of_camera_t *cam, const of_depth_filter_params_t *p,
@@ -214,23 +308,10 @@ extern "C" of_status_t of_depth_filter(const of_camera_t *cam, const of_depth_fi
   if (k > 1 || d_in == d_out) {
     if (!d_scratch || d_scratch == d_in || d_scratch == d_out) return OF_ERR_INVALID_ARGUMENT;
   }
-  // ping-pong between d_scratch and d_out so that the last step writes d_out;
-  // an in-place chain starts from a copy of the input in d_scratch
-  const uint16_t *src = d_in;
-  if (d_in == d_out) {
+  // (in place: blocks read their neighbours' input, so from a copy)
+  if (d_in == d_out)
     OF_CUDA_TRY(cudaMemcpyAsync(d_scratch, d_in, bytes, cudaMemcpyDeviceToDevice, s));
-    src = d_scratch;
-  }
-  for (int i = 0; i < k; ++i) {
-    const int left = k - 1 - i;  // steps after this one
-    uint16_t *dst = (left % 2 == 0) ? d_out : d_scratch;
-    if (dst == src) dst = (dst == d_out) ? d_scratch : d_out;
-    of_status_t st = launch_step(steps[i], cam, p, src, dst, s);
-    if (st != OF_OK) return st;
-    src = dst;
-  }
-  if (src != d_out) OF_CUDA_TRY(cudaMemcpyAsync(d_out, src, bytes, cudaMemcpyDeviceToDevice, s));
-  return OF_OK;
+  return launch_chain(steps, k, cam, p, d_in == d_out ? d_scratch : d_in, d_out, s);
 }
 
 extern "C" void of_depth_filter_defaults(of_depth_filter_params_t *p) {
