@@ -11,6 +11,8 @@
 // (ICP.cpp:174) is applied on the fly inside the ICP kernel instead.
 #include "of_batch.cuh"
 
+#include <type_traits>
+
 using namespace of;
 
 bool of_camera_valid(const of_camera_t *c);
@@ -28,120 +30,163 @@ __device__ __forceinline__ bool depth_valid(float d, float dmin, float dmax) {
 // Bilateral filter of the raw uint16 depth. Invalid centre -> 0; invalid
 // neighbours get weight 0. Weight = 2^-(r^2 ks + delta^2 kr) with
 // ks = log2(e)/(2 sigma_s^2), kr = log2(e)/(2 sigma_r^2).
-__global__ void __launch_bounds__(256) k_bilateral(const uint16_t *__restrict__ depth, int pitch,
-                                                   int w, int h, float dmin, float dmax, int R,
-                                                   float ks, float kr, float *__restrict__ out) {
-  extern __shared__ float tile[];
-  const int tw = kTileX + 2 * R;
-  const int th = kTileY + 2 * R;
-  const int x0 = blockIdx.x * kTileX - R;
-  const int y0 = blockIdx.y * kTileY - R;
-  for (int i = threadIdx.x; i < tw * th; i += blockDim.x) {
-    int tx = i % tw, ty = i / tw;
-    int gx = x0 + tx, gy = y0 + ty;
-    float d = 0.f;
-    if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-      d = (float)__ldg(depth + (size_t)gy * pitch + gx);
-      if (!depth_valid(d, dmin, dmax)) d = 0.f;
-    }
-    tile[i] = d;
-  }
-  __syncthreads();
-  const int lx = threadIdx.x % kTileX, ly = threadIdx.x / kTileX;
-  const int x = blockIdx.x * kTileX + lx, y = blockIdx.y * kTileY + ly;
-  if (x >= w || y >= h) return;
-  const float c = tile[(ly + R) * tw + lx + R];
-  float result = 0.f;
-  if (c > 0.f) {
-    float sw = 0.f, sd = 0.f;
-    for (int dy = -R; dy <= R; ++dy) {
-      const float *row = tile + (ly + R + dy) * tw + lx + R;
-      const float ry = (float)(dy * dy) * ks;
-      for (int dx = -R; dx <= R; ++dx) {
-        float q = row[dx];
-        float del = q - c;
-        float e = fmaf(del * del, kr, fmaf((float)(dx * dx), ks, ry));
-        float wt = q > 0.f ? exp2f(-e) : 0.f;
-        sw += wt;
-        sd = fmaf(wt, q, sd);
-      }
-    }
-    result = sd / sw;
-  }
-  out[(size_t)y * w + x] = result;
-}
-
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
-// Same filter with the radius fixed at compile time (taps fully unrolled).
-// Invalid depths are stored as -1e30 in the tile: their squared range
-// difference overflows to +inf and their weight 2^-inf is exactly 0, so no
-// per-tap select is needed. One ex2 per tap.
-// (tile (bx, by) of the image; the kernels below pass their block index)
-template <int R, bool UNROLL_ROWS>
-__device__ __forceinline__ void bilateral_tile(const uint16_t *__restrict__ depth, int pitch,
-                                               int w, int h, float dmin, float dmax, float ks,
-                                               float kr, float *__restrict__ out, int bx, int by) {
-  constexpr int TW = kTileX + 2 * R;
-  constexpr int TH = kTileY + 2 * R;
-  __shared__ float tile[TH * TW];
-  const int x0 = bx * kTileX - R;
-  const int y0 = by * kTileY - R;
-  for (int i = threadIdx.x; i < TW * TH; i += blockDim.x) {
-    int tx = i % TW, ty = i / TW;
-    int gx = x0 + tx, gy = y0 + ty;
-    float d = -1e30f;
-    if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-      float v = (float)__ldg(depth + (size_t)gy * pitch + gx);
-      if (depth_valid(v, dmin, dmax)) d = v;
-    }
-    tile[i] = d;
-  }
-  __syncthreads();
-  const int lx = threadIdx.x % kTileX, ly = threadIdx.x / kTileX;
-  const int x = bx * kTileX + lx, y = by * kTileY + ly;
-  if (x >= w || y >= h) return;
-  const float *ctr = tile + (ly + R) * TW + lx + R;
-  const float c = *ctr;
-  float result = 0.f;
-  if (c > 0.f) {
-    const float nkr = -kr;
-    float sw = 0.f, sd = 0.f;
-    // single-stream filter: rows not unrolled (32 registers a thread, see
-    // filter_footprint); the batched one unrolls them (the same sums)
-    auto row = [&](int dy) {
-      const float ry = -(float)(dy * dy) * ks;
-#pragma unroll
-      for (int dx = -R; dx <= R; ++dx) {
-        float q = ctr[dy * TW + dx];
-        float del = q - c;
-        float e = fmaf(del * nkr, del, fmaf(-(float)(dx * dx), ks, ry));
-        float wt = ex2_approx(e);
-        sw += wt;
-        sd = fmaf(wt, q, sd);
-      }
-    };
-    if (UNROLL_ROWS) {
-#pragma unroll
-      for (int dy = -R; dy <= R; ++dy) row(dy);
-    } else {
-#pragma unroll 1
-      for (int dy = -R; dy <= R; ++dy) row(dy);
-    }
-    result = sd / sw;
-  }
-  out[(size_t)y * w + x] = result;
+// Two FP32 values an instruction (each half rounded as the scalar form rounds).
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 z, x, y; "
+      "mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 z, x, y; "
+      "mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{.reg .b64 x, y, z, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; "
+      "fma.rn.f32x2 w, x, y, z; mov.b64 {%0, %1}, w;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
 }
 
-template <int R>
-__global__ void __launch_bounds__(256) k_bilateral_r(const uint16_t *__restrict__ depth, int pitch,
-                                                     int w, int h, float dmin, float dmax,
-                                                     float ks, float kr, float *__restrict__ out) {
-  bilateral_tile<R, false>(depth, pitch, w, h, dmin, dmax, ks, kr, out, blockIdx.x, blockIdx.y);
+// The radius is fixed at compile time. Invalid depths are stored as -1e30 in
+// the tile: their squared range difference overflows to +inf and their weight
+// 2^-inf is exactly 0, so no per-tap select is needed. One ex2 per tap: the special-function unit (16 a clock and SM) is the bound,
+// 24.6 us for the 361 taps of a 640x480 image. A thread owns two pixels, one
+// above the other, and forms both their weights for a tile value with paired
+// FP32 instructions, so the taps take half of the issue slots and leave the
+// rest to the blocks that share the SM (the fusion of the previous frame runs
+// beside this filter). The tile holds each value twice, one 8-byte read a
+// pair. Every pixel adds its taps in row order, as with a thread a pixel.
+// Measured at 640x480, sigma 4.5 px (R = 9): a thread a pixel 41.9 us, two a
+// thread 35 us.
+// PX = 1 is the thread-a-pixel form, for images too small to fill the SMs with
+// pairs. (tile (bx, by) of 32 x PX TY pixels; 32 TY threads)
+// The radii 3..10 and 12 evaluate the exponent and 2^x in the form above; the
+// others (FULL: 1, 2, 11, 13..16) keep the signs and the full-range exp2f that
+// they always had.
+constexpr bool full_form(int R) { return R < 3 || R == 11 || R > 12; }
+template <int R, int TY, int PX>
+struct BilateralTile {
+  static constexpr int TW = kTileX + 2 * R, TH = PX * TY + 2 * R;
+  using Q = std::conditional_t<PX == 2, float2, float>;
+  Q q[TH * TW];                                        // {d, d}, or d
+  float2 base[PX == 2 ? (2 * R + 2) * (R + 1) : 1];    // row y (of both pixels' rows), |dx|
+};
+__device__ __forceinline__ float lower(float v) { return v; }
+__device__ __forceinline__ float lower(float2 v) { return v.x; }
+template <int R, int TY, int PX>
+__device__ __forceinline__ void bilateral_tile(BilateralTile<R, TY, PX> &S,
+                                               const uint16_t *__restrict__ depth, int pitch, int w,
+                                               int h, float dmin, float dmax, float ks, float kr,
+                                               float *__restrict__ out, int bx, int by) {
+  constexpr int TW = BilateralTile<R, TY, PX>::TW, TH = BilateralTile<R, TY, PX>::TH;
+  const int x0 = bx * kTileX - R;
+  const int y0 = by * PX * TY - R;
+  // the pyramid may be launched now (it waits for this grid before reading)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  constexpr bool FULL = full_form(R);
+  constexpr float sg = FULL ? 1.f : -1.f;
+  for (int i = threadIdx.x; i < TW * TH; i += 32 * TY) {
+    const int gx = x0 + i % TW, gy = y0 + i / TW;
+    float d = FULL ? 0.f : -1e30f;
+    if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
+      const float v = (float)__ldg(depth + (size_t)gy * pitch + gx);
+      if (depth_valid(v, dmin, dmax)) d = v;
+    }
+    if constexpr (PX == 2) S.q[i] = make_float2(d, d);
+    else S.q[i] = d;
+  }
+  // the spatial exponents: tile row r (0 .. 2R + 1) lies r - R below the upper
+  // pixel and r - R - 1 below the lower one
+  for (int i = threadIdx.x; PX == 2 && i < (2 * R + 2) * (R + 1); i += 32 * TY) {
+    const int r = i / (R + 1), dx = i % (R + 1), d0 = r - R, d1 = r - R - 1;
+    const float r0 = __fmul_rn(sg * (float)(d0 * d0), ks), r1 = __fmul_rn(sg * (float)(d1 * d1), ks);
+    S.base[i] = make_float2(fmaf(sg * (float)(dx * dx), ks, r0), fmaf(sg * (float)(dx * dx), ks, r1));
+  }
+  __syncthreads();
+  const int lx = threadIdx.x % kTileX, ly = PX * (threadIdx.x / kTileX);
+  const int x = bx * kTileX + lx, y = by * PX * TY + ly;
+  if (x >= w || y >= h) return;
+  const auto *row = S.q + ly * TW + lx + R;  // row 0 of the pixels' rows
+  const float2 c = make_float2(lower(row[R * TW]), PX == 2 ? lower(row[(R + PX - 1) * TW]) : -1.f);
+  float2 res = make_float2(0.f, 0.f);
+  if (c.x > 0.f || c.y > 0.f) {
+    const float2 nc = make_float2(-c.x, -c.y), nkr = make_float2(-kr, -kr);
+    float2 sw = make_float2(0.f, 0.f), sd = sw;
+    // row 0 reaches the upper pixel only, row 2R + 1 the lower one only
+    // row r for one pixel (rounded products: the compiler must not regroup them,
+    // so that both forms give the same bits)
+    auto single = [&](int r, bool low) {
+      const auto *q = row + r * TW;
+      const int d = low ? r - R - 1 : r - R;
+      const float ry = __fmul_rn(sg * (float)(d * d), ks);
+#pragma unroll
+      for (int dx = -R; dx <= R; ++dx) {
+        const float v = lower(q[dx]), del = v + (low ? nc.y : nc.x);
+        const float b0 = fmaf(sg * (float)(dx * dx), ks, ry);
+        float wt;
+        if (FULL) {
+          wt = exp2f(-fmaf(del * del, kr, b0));
+          wt = v > 0.f ? wt : 0.f;
+        } else {
+          wt = ex2_approx(fmaf(__fmul_rn(del, -kr), del, b0));
+        }
+        if (low) { sw.y += wt; sd.y = fmaf(wt, v, sd.y); }
+        else { sw.x += wt; sd.x = fmaf(wt, v, sd.x); }
+      }
+    };
+    if constexpr (PX == 1) {
+#pragma unroll 1
+      for (int r = 0; r <= 2 * R; ++r) single(r, false);
+    } else {
+      single(0, false);
+#pragma unroll 1
+      for (int r = 1; r <= 2 * R; ++r) {
+        const float2 *q = row + r * TW, *base = S.base + r * (R + 1);
+#pragma unroll
+        for (int dx = -R; dx <= R; ++dx) {
+          const float2 v = q[dx];
+          const float2 del = add2(v, nc);
+          float2 wt;
+          if (FULL) {
+            const float2 e = fma2(mul2(del, del), make_float2(kr, kr), base[dx < 0 ? -dx : dx]);
+            wt = make_float2(exp2f(-e.x), exp2f(-e.y));
+            if (!(v.x > 0.f)) wt = make_float2(0.f, 0.f);
+          } else {
+            const float2 e = fma2(mul2(del, nkr), del, base[dx < 0 ? -dx : dx]);
+            wt = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+          }
+          sw = add2(sw, wt);
+          sd = fma2(wt, v, sd);
+        }
+      }
+      single(2 * R + 1, true);
+    }
+    if (c.x > 0.f) res.x = sd.x / sw.x;
+    if (c.y > 0.f) res.y = sd.y / sw.y;
+  }
+  out[(size_t)y * w + x] = res.x;
+  if (PX == 2 && y + 1 < h) out[(size_t)(y + 1) * w + x] = res.y;
+}
+
+template <int R, int TY, int PX>
+__global__ void __launch_bounds__(32 * TY) k_bilateral_r(const uint16_t *__restrict__ depth, int pitch,
+                                                         int w, int h, float dmin, float dmax,
+                                                         float ks, float kr,
+                                                         float *__restrict__ out) {
+  __shared__ BilateralTile<R, TY, PX> S;
+  bilateral_tile<R, TY, PX>(S, depth, pitch, w, h, dmin, dmax, ks, kr, out, blockIdx.x, blockIdx.y);
 }
 
 // No filter: the raw depth as float, invalid -> 0 (the reference converts the
@@ -160,24 +205,99 @@ __global__ void k_depth_raw(const uint16_t *__restrict__ depth, int pitch, int w
   depth_raw_tile(depth, pitch, w, h, dmin, dmax, out, blockIdx.x, blockIdx.y);
 }
 
-// Level l -> l+1: pixel (x, y) averages the valid pixels of the 2x2 block
+// Every pyramid level and its vertex / normal map in one launch: a block holds
+// 32 x 32 pixels of the filtered depth, and as much to the right and below as
+// the next levels' neighbours need (8 pixels with four levels), in shared
+// memory, halves it level by level there, and writes each level's depth and
+// points. Bound by the 32 bytes a pixel of the points. (As a launch a level
+// and a map, 5 at three levels: 13.6 us at 640x480 and their gaps, now 6.5.)
+//
+// Level l -> l + 1: pixel (x, y) averages the valid pixels of the 2x2 block
 // {2x, 2x+1} x {2y, 2y+1} that lie within 3 sigma_r of the block's first
-// valid pixel (row-major order); 0 if the block has none.
-__device__ __forceinline__ void pyr_down_tile(const float *__restrict__ src, int sw, int sh,
-                                              float *__restrict__ dst, int dw, int dh, float guard,
-                                              int bx, int by) {
-  int x = bx * blockDim.x + threadIdx.x;
-  int y = by * blockDim.y + threadIdx.y;
-  if (x >= dw || y >= dh) return;
-  float ref = 0.f, sum = 0.f;
-  int cnt = 0;
+// valid pixel (row-major order); 0 if the block has none. Pixels outside the
+// image hold 0, which is invalid.
+struct PyrLevel {
+  float *depth;
+  float4 *pts;
+  int w, h;
+  float cx, cy, ifx, ify;
+};
+struct PyrMaps {
+  PyrLevel lv[kMaxLevels];
+  int levels;
+  bool wide;  // the points are 32-byte aligned: one store a pixel
+};
+constexpr int kPyrTile = 32, kPyrThreads = 256;
+constexpr int pyr_edge(int l) { return (kPyrTile >> l) + (8 >> l); }  // tile edge at level l
+struct PyrSmem {
+  float d0[pyr_edge(0) * pyr_edge(0)], d1[pyr_edge(1) * pyr_edge(1)], d2[pyr_edge(2) * pyr_edge(2)],
+      d3[pyr_edge(3) * pyr_edge(3)];
+};
+
+// Camera-space vertex and normal of pixel (x, y) from its depth d and the
+// depths to its right and below (0 where there is none). Differences of
+// neighbouring vertices are formed from depth differences (no cancellation
+// between large coordinates).
+__device__ __forceinline__ void put_point(const PyrLevel &L, bool wide, int x, int y, float d,
+                                          float d10, float d01) {
+  const size_t p = (size_t)y * L.w + x;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float ifx = L.ifx, ify = L.ify;
+  if (d > 0.f) {
+    float ax = (float)x - L.cx, ay = (float)y - L.cy;
+    v = make_float4(-d * ax * ifx, -d * ay * ify, -d, 1.f);
+    if (d10 > 0.f && d01 > 0.f) {
+      float e10 = d10 - d, e01 = d01 - d;
+      float3 a = make_float3(-ifx * fmaf(e10, ax, d10), -ify * ay * e10, -e10);
+      float3 b = make_float3(-ifx * ax * e01, -ify * fmaf(e01, ay, d01), -e01);
+      float3 c = make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+      float l2 = c.x * c.x + c.y * c.y + c.z * c.z;
+      if (l2 > 0.f) {
+        float il = rsqrtf(l2);
+        il = il * (1.5f - 0.5f * l2 * il * il);  // one Newton step on rsqrt
+        n = make_float4(c.x * il, c.y * il, c.z * il, 1.f);
+      }
+    }
+  }
+  if (wide) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(L.pts + 2 * p),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "f"(n.x), "f"(n.y), "f"(n.z), "f"(n.w)
+                 : "memory");
+  } else {
+    L.pts[2 * p] = v;
+    L.pts[2 * p + 1] = n;
+  }
+}
+
+// level l of the block: its points, from the tile of its depths
+template <int L>
+__device__ __forceinline__ void put_level(const PyrMaps &M, const float *__restrict__ d, int bx,
+                                          int by) {
+  constexpr int E = pyr_edge(L), N = kPyrTile >> L;
+  const int x0 = bx * N, y0 = by * N;
+  for (int i = threadIdx.x; i < N * N; i += kPyrThreads) {
+    const int tx = i % N, ty = i / N;
+    if (x0 + tx >= M.lv[L].w || y0 + ty >= M.lv[L].h) continue;
+    const float *c = d + ty * E + tx;
+    put_point(M.lv[L], M.wide, x0 + tx, y0 + ty, c[0], c[1], c[E]);
+  }
+}
+// the tile of level L + 1 from that of level L
+template <int L>
+__device__ __forceinline__ void halve(const PyrMaps &M, const float *__restrict__ src,
+                                      float *__restrict__ dst, float guard, int bx, int by) {
+  constexpr int E = pyr_edge(L), F = pyr_edge(L + 1), N = kPyrTile >> (L + 1);
+  const PyrLevel &T = M.lv[L + 1];
+  for (int i = threadIdx.x; i < F * F; i += kPyrThreads) {
+    const int tx = i % F, ty = i / F;
+    float ref = 0.f, sum = 0.f;
+    int cnt = 0;
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      int sx = 2 * x + i, sy = 2 * y + j;
-      if (sx < sw && sy < sh) {
-        float d = src[(size_t)sy * sw + sx];
+      for (int k = 0; k < 2; ++k) {
+        const float d = src[(2 * ty + j) * E + 2 * tx + k];
         if (d > 0.f) {
           if (cnt == 0) ref = d;
           if (fabsf(d - ref) <= guard) {
@@ -186,53 +306,52 @@ __device__ __forceinline__ void pyr_down_tile(const float *__restrict__ src, int
           }
         }
       }
-    }
-  dst[(size_t)y * dw + x] = cnt ? sum / (float)cnt : 0.f;
+    const float v = cnt ? sum / (float)cnt : 0.f;
+    dst[i] = v;
+    const int x = bx * N + tx, y = by * N + ty;
+    if (tx < N && ty < N && x < T.w && y < T.h) T.depth[(size_t)y * T.w + x] = v;
+  }
 }
-__global__ void k_pyr_down(const float *__restrict__ src, int sw, int sh, float *__restrict__ dst,
-                           int dw, int dh, float guard) {
-  pyr_down_tile(src, sw, sh, dst, dw, dh, guard, blockIdx.x, blockIdx.y);
+__device__ __forceinline__ void pyramid_tile(PyrSmem &S, const PyrMaps &M, float guard, int bx, int by) {
+  constexpr int E = pyr_edge(0);
+  const PyrLevel &T = M.lv[0];
+  for (int i = threadIdx.x; i < E * E; i += kPyrThreads) {
+    const int x = bx * kPyrTile + i % E, y = by * kPyrTile + i / E;
+    S.d0[i] = x < T.w && y < T.h ? T.depth[(size_t)y * T.w + x] : 0.f;
+  }
+  __syncthreads();
+  if (M.levels > 1) halve<0>(M, S.d0, S.d1, guard, bx, by);
+  put_level<0>(M, S.d0, bx, by);
+  if (M.levels < 2) return;
+  __syncthreads();
+  if (M.levels > 2) halve<1>(M, S.d1, S.d2, guard, bx, by);
+  put_level<1>(M, S.d1, bx, by);
+  if (M.levels < 3) return;
+  __syncthreads();
+  if (M.levels > 3) halve<2>(M, S.d2, S.d3, guard, bx, by);
+  put_level<2>(M, S.d2, bx, by);
+  if (M.levels < 4) return;
+  __syncthreads();
+  put_level<3>(M, S.d3, bx, by);
+}
+__global__ void __launch_bounds__(kPyrThreads) k_pyramid(PyrMaps M, float guard) {
+  __shared__ PyrSmem S;
+  // (a programmatic launch starts before the filter has finished)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pyramid_tile(S, M, guard, blockIdx.x, blockIdx.y);
 }
 
-// Camera-space vertex and normal of every pixel of one level. Differences
-// of neighbouring vertices are formed from depth differences (no
-// cancellation between large coordinates).
-__device__ __forceinline__ void vertex_normal_tile(const float *__restrict__ depth, int w, int h,
-                                                   float cx, float cy, float ifx, float ify,
-                                                   float4 *__restrict__ pts, int bx, int by) {
-  int x = bx * blockDim.x + threadIdx.x;
-  int y = by * blockDim.y + threadIdx.y;
-  if (x >= w || y >= h) return;
-  size_t p = (size_t)y * w + x;
-  float d = depth[p];
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (d > 0.f) {
-    float ax = (float)x - cx, ay = (float)y - cy;
-    v = make_float4(-d * ax * ifx, -d * ay * ify, -d, 1.f);
-    if (x + 1 < w && y + 1 < h) {
-      float d10 = depth[p + 1];
-      float d01 = depth[p + w];
-      if (d10 > 0.f && d01 > 0.f) {
-        float e10 = d10 - d, e01 = d01 - d;
-        float3 a = make_float3(-ifx * fmaf(e10, ax, d10), -ify * ay * e10, -e10);
-        float3 b = make_float3(-ifx * ax * e01, -ify * fmaf(e01, ay, d01), -e01);
-        float3 c = make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-        float l2 = c.x * c.x + c.y * c.y + c.z * c.z;
-        if (l2 > 0.f) {
-          float il = rsqrtf(l2);
-          il = il * (1.5f - 0.5f * l2 * il * il);  // one Newton step on rsqrt
-          n = make_float4(c.x * il, c.y * il, c.z * il, 1.f);
-        }
-      }
-    }
+// the levels of the frame pyramid at `base`
+PyrMaps pyramid_maps(const of_camera_t &cam, const of_pyramid_layout_t &lay, int levels, char *base) {
+  PyrMaps M = {};
+  M.levels = levels;
+  M.wide = ((uintptr_t)base & 31u) == 0;  // (a level's points start at a multiple of 256 bytes)
+  for (int l = 0; l < levels; ++l) {
+    const of_camera_t c = camera_level(cam, l);
+    M.lv[l] = {(float *)(base + lay.depth_offset[l]), (float4 *)(base + lay.points_offset[l]),
+               c.width, c.height, c.cx, c.cy, (float)(1.0 / (double)c.fx), (float)(1.0 / (double)c.fy)};
   }
-  pts[2 * p] = v;
-  pts[2 * p + 1] = n;
-}
-__global__ void k_vertex_normal(const float *__restrict__ depth, int w, int h, float cx, float cy,
-                                float ifx, float ify, float4 *__restrict__ pts) {
-  vertex_normal_tile(depth, w, h, cx, cy, ifx, ify, pts, blockIdx.x, blockIdx.y);
+  return M;
 }
 
 // ---------------------------------------------------------------- batched --
@@ -245,41 +364,33 @@ struct FilterJob {
   float *out;
 };
 struct PyrJob {
-  const float *src;
-  float *dst;
-  int sw, sh, dw, dh, gx;
-};
-struct VnJob {
-  const float *depth;
-  float4 *pts;
-  int w, h, gx;
-  float cx, cy, ifx, ify;
+  PyrMaps maps;
+  int gx;
 };
 
+constexpr int kBatchTy = 4;
 template <int R>
-__global__ void __launch_bounds__(256) k_bilateral_batch(const FilterJob *__restrict__ jobs,
-                                                         const int *__restrict__ first, int n,
-                                                         int parity, float ks, float kr) {
+__global__ void __launch_bounds__(32 * kBatchTy) k_bilateral_batch(const FilterJob *__restrict__ jobs,
+                                                                   const int *__restrict__ first,
+                                                                   int n, int parity, float ks,
+                                                                   float kr) {
+  __shared__ BilateralTile<R, kBatchTy, 2> S;
   const int j = batch_job(first, n, blockIdx.x);
   const FilterJob &J = jobs[j];
   const int b = blockIdx.x - __ldg(first + j);
-  bilateral_tile<R, true>(J.depth[parity], J.pitch, J.w, J.h, J.dmin, J.dmax, ks, kr, J.out, b % J.gx,
-                    b / J.gx);
+  bilateral_tile<R, kBatchTy, 2>(S, J.depth[parity], J.pitch, J.w, J.h, J.dmin, J.dmax, ks, kr, J.out,
+                              b % J.gx, b / J.gx);
 }
-// The single-stream filter runs on the step graph's pre-processing branch, at
-// the lower stream priority, beside the integration and the raycast. A block of it that
-// sits on an SM holds registers and threads that their blocks then wait for,
-// so the filter keeps a small footprint: 32 registers a thread and at most
-// kFilterBlocksPerSm blocks per SM, set by a reservation of dynamic shared
-// memory that the kernel leaves unused. Measured at C2 (300 frames, alternating
-// runs on one B200): fully unrolled rows (128 registers, two blocks filling
-// the register file) 2956 / 2903-2916 frames/s (value / e2e); 32 registers
-// and two blocks per SM 3008 / 2941-2946; three per SM 2964-2967; one per SM
-// gained `value` but lost `e2e` (the branch then took 108 us); 32 registers
-// with no cap (eight per SM) lost 3 %. The filtered depth is the same bits.
-// (The batched filter keeps the unrolled rows and no cap: capped the same way
-// it lost 5 % of the 64-stream batch's frames/s.)
-constexpr int kFilterBlocksPerSm = 2;
+// In a step graph the single-stream filter runs on the pre-processing branch,
+// at the lower stream priority, beside the integration and the raycast. A
+// block of it that sits on an SM holds registers and threads that their blocks
+// then wait for, so a captured filter keeps a small footprint: at most
+// kFilterBlocksPerSm blocks (of 128 threads) per SM, set by a reservation of
+// dynamic shared memory that the kernel leaves unused. Measured at C2 (us a
+// tracked frame, frame in, pose out): no cap 319.0; 2 / 3 / 4 / 6 blocks 322.2
+// / 313.6 / 315.7 / 325.3; blocks of 256 threads, at most 2: 314.5. A call
+// outside a capture runs by itself and takes every SM.
+constexpr int kFilterBlocksPerSm = 3;
 template <typename Kernel>
 cudaError_t filter_footprint(Kernel *k, size_t *dyn) {
   int dev = 0, smem_sm = 0, reserved = 0;
@@ -305,19 +416,35 @@ __global__ void k_depth_raw_batch(const FilterJob *__restrict__ jobs, const int 
   const int b = blockIdx.x - __ldg(first + j);
   depth_raw_tile(J.depth[parity], J.pitch, J.w, J.h, J.dmin, J.dmax, J.out, b % J.gx, b / J.gx);
 }
-__global__ void k_pyr_down_batch(const PyrJob *__restrict__ jobs, const int *__restrict__ first,
-                                 int n, float guard) {
+__global__ void __launch_bounds__(kPyrThreads) k_pyramid_batch(const PyrJob *__restrict__ jobs,
+                                                               const int *__restrict__ first, int n,
+                                                               float guard) {
+  __shared__ PyrSmem S;
   const int j = batch_job(first, n, blockIdx.x);
   const PyrJob &J = jobs[j];
   const int b = blockIdx.x - __ldg(first + j);
-  pyr_down_tile(J.src, J.sw, J.sh, J.dst, J.dw, J.dh, guard, b % J.gx, b / J.gx);
+  pyramid_tile(S, J.maps, guard, b % J.gx, b / J.gx);
 }
-__global__ void k_vertex_normal_batch(const VnJob *__restrict__ jobs, const int *__restrict__ first,
-                                      int n) {
-  const int j = batch_job(first, n, blockIdx.x);
-  const VnJob &J = jobs[j];
-  const int b = blockIdx.x - __ldg(first + j);
-  vertex_normal_tile(J.depth, J.w, J.h, J.cx, J.cy, J.ifx, J.ify, J.pts, b % J.gx, b / J.gx);
+
+// Launches the filter of one image.
+template <int R>
+of_status_t launch_bilateral(const uint16_t *depth, int pitch, int w, int h, float dmin, float dmax,
+                             float ks, float kr, float *out, cudaStream_t s, bool captured) {
+  const int gx = (w + kTileX - 1) / kTileX;
+  // blocks of 32 x 8 pixels, two a thread (640x480 pyramid with blocks of 32 x
+  // 16 / 8 / 4 / 2: 47.3 / 45.2 / 47.3 / 48.9 us: finer ones even out the last
+  // wave, but load more halo); a pixel a thread, a warp a block, while the
+  // larger ones would not give every SM two (160x120: 19.2 against 16.4 us)
+  if ((long)gx * ((h + 7) / 8) >= 2 * kSmCount) {
+    size_t dyn = 0;
+    const cudaError_t e = captured ? filter_footprint(k_bilateral_r<R, 4, 2>, &dyn) : cudaSuccess;
+    if (e != cudaSuccess) return of_set_cuda_error(e);
+    k_bilateral_r<R, 4, 2><<<dim3(gx, (h + 7) / 8), 128, dyn, s>>>(depth, pitch, w, h, dmin, dmax, ks, kr,
+                                                                out);
+  } else {
+    k_bilateral_r<R, 1, 1><<<dim3(gx, h), 32, 0, s>>>(depth, pitch, w, h, dmin, dmax, ks, kr, out);
+  }
+  return of_launch_status();
 }
 
 int filter_radius(const of_filter_params_t *fp) {
@@ -328,29 +455,23 @@ int filter_radius(const of_filter_params_t *fp) {
 
 namespace of {
 
-// Level-0 filter of every stream in one launch, then one launch per pyramid
-// level, then the vertex/normal maps of every (stream, level) in one launch.
+// Level-0 filter of every stream in one launch, then every stream's pyramid
+// levels and maps in another.
 struct PreprocessBatch {
   int n = 0, levels = 0, radius = 0;
   float ks = 0.f, kr = 0.f, guard = 0.f;
   FilterJob *filter = nullptr;
   int *filter_first = nullptr, filter_blocks = 0;
-  PyrJob *pyr[kMaxLevels] = {};
-  int *pyr_first[kMaxLevels] = {}, pyr_blocks[kMaxLevels] = {};
-  VnJob *vn = nullptr;
-  int *vn_first = nullptr, vn_jobs = 0, vn_blocks = 0;
+  PyrJob *pyr = nullptr;
+  int *pyr_first = nullptr, pyr_blocks = 0;
 };
 
 void preprocess_batch_destroy(PreprocessBatch *b) {
   if (!b) return;
   cudaFree(b->filter);
   cudaFree(b->filter_first);
-  for (int l = 0; l < kMaxLevels; ++l) {
-    cudaFree(b->pyr[l]);
-    cudaFree(b->pyr_first[l]);
-  }
-  cudaFree(b->vn);
-  cudaFree(b->vn_first);
+  cudaFree(b->pyr);
+  cudaFree(b->pyr_first);
   delete b;
 }
 
@@ -373,10 +494,11 @@ of_status_t preprocess_batch_create(const BatchStream *s, int n, const BatchPara
   b->guard = 3.0f * fp->sigma_range_mm;
   FilterJob *fj = new FilterJob[n];
   PyrJob *pj = new PyrJob[n];
-  VnJob *vj = new VnJob[(size_t)n * fp->levels];
-  int *first = new int[(size_t)n * fp->levels + 1];
+  int *first = new int[n + 1];
   of_status_t st = OF_OK;
-  // level-0 filter (32x8 tiles either way)
+  // level-0 filter: 32 x 8 tiles either way
+  static_assert(kTileY == 2 * kBatchTy, "one tile grid");
+  const int rows = kTileY;
   first[0] = 0;
   for (int i = 0; i < n && st == OF_OK; ++i) {
     of_pyramid_layout_t lay;
@@ -385,48 +507,26 @@ of_status_t preprocess_batch_create(const BatchStream *s, int n, const BatchPara
     fj[i] = {{s[i].depth[0], s[i].depth[1]}, w, w, h, (w + kTileX - 1) / kTileX,
              s[i].cam.min_depth_mm, s[i].cam.max_depth_mm,
              (float *)((char *)s[i].frame + lay.depth_offset[0])};
-    first[i + 1] = first[i] + fj[i].gx * ((h + kTileY - 1) / kTileY);
+    first[i + 1] = first[i] + fj[i].gx * ((h + rows - 1) / rows);
   }
   if (st == OF_OK) {
     b->filter_blocks = first[n];
     st = upload_jobs(fj, first, n, &b->filter, &b->filter_first);
   }
-  for (int l = 1; l < fp->levels && st == OF_OK; ++l) {
-    first[0] = 0;
-    for (int i = 0; i < n; ++i) {
-      of_pyramid_layout_t lay;
-      of_pyramid_layout(&s[i].cam, fp->levels, &lay);
-      char *base = (char *)s[i].frame;
-      pj[i] = {(const float *)(base + lay.depth_offset[l - 1]), (float *)(base + lay.depth_offset[l]),
-               lay.width[l - 1], lay.height[l - 1], lay.width[l], lay.height[l],
-               (lay.width[l] + 31) / 32};
-      first[i + 1] = first[i] + pj[i].gx * ((lay.height[l] + 7) / 8);
-    }
-    b->pyr_blocks[l] = first[n];
-    st = upload_jobs(pj, first, n, &b->pyr[l], &b->pyr_first[l]);
-  }
   if (st == OF_OK) {
-    int k = 0;
     first[0] = 0;
     for (int i = 0; i < n; ++i) {
       of_pyramid_layout_t lay;
       of_pyramid_layout(&s[i].cam, fp->levels, &lay);
-      char *base = (char *)s[i].frame;
-      for (int l = 0; l < fp->levels; ++l, ++k) {
-        const of_camera_t c = camera_level(s[i].cam, l);
-        vj[k] = {(const float *)(base + lay.depth_offset[l]), (float4 *)(base + lay.points_offset[l]),
-                 c.width, c.height, (c.width + 31) / 32, c.cx, c.cy,
-                 (float)(1.0 / (double)c.fx), (float)(1.0 / (double)c.fy)};
-        first[k + 1] = first[k] + vj[k].gx * ((c.height + 7) / 8);
-      }
+      pj[i].maps = pyramid_maps(s[i].cam, lay, fp->levels, (char *)s[i].frame);
+      pj[i].gx = (s[i].cam.width + kPyrTile - 1) / kPyrTile;
+      first[i + 1] = first[i] + pj[i].gx * ((s[i].cam.height + kPyrTile - 1) / kPyrTile);
     }
-    b->vn_jobs = k;
-    b->vn_blocks = first[k];
-    st = upload_jobs(vj, first, k, &b->vn, &b->vn_first);
+    b->pyr_blocks = first[n];
+    st = upload_jobs(pj, first, n, &b->pyr, &b->pyr_first);
   }
   delete[] fj;
   delete[] pj;
-  delete[] vj;
   delete[] first;
   if (st != OF_OK) {
     preprocess_batch_destroy(b);
@@ -443,7 +543,7 @@ of_status_t preprocess_batch_launch(const PreprocessBatch *b, int parity, cudaSt
   } else {
 #define OF_BILATERAL_BATCH(RR)                                                          \
   case RR:                                                                              \
-    k_bilateral_batch<RR><<<b->filter_blocks, kTileX * kTileY, 0, s>>>(                 \
+    k_bilateral_batch<RR><<<b->filter_blocks, 32 * kBatchTy, 0, s>>>(                 \
         b->filter, b->filter_first, b->n, parity, b->ks, b->kr);                        \
     break;
     switch (b->radius) {
@@ -461,10 +561,7 @@ of_status_t preprocess_batch_launch(const PreprocessBatch *b, int parity, cudaSt
     }
 #undef OF_BILATERAL_BATCH
   }
-  for (int l = 1; l < b->levels; ++l)
-    k_pyr_down_batch<<<b->pyr_blocks[l], dim3(32, 8), 0, s>>>(b->pyr[l], b->pyr_first[l], b->n,
-                                                              b->guard);
-  k_vertex_normal_batch<<<b->vn_blocks, dim3(32, 8), 0, s>>>(b->vn, b->vn_first, b->vn_jobs);
+  k_pyramid_batch<<<b->pyr_blocks, kPyrThreads, 0, s>>>(b->pyr, b->pyr_first, b->n, b->guard);
   return of_launch_status();
 }
 
@@ -485,30 +582,30 @@ extern "C" of_status_t of_preprocess(const of_camera_t *cam, const of_filter_par
   of_status_t st = of_pyramid_layout(cam, fp->levels, &lay);
   if (st != OF_OK) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  // (a stream whose status cannot be read is taken as captured)
+  const bool captured = cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
   char *base = (char *)d_frame;
   const double log2e = 1.4426950408889634;
   float ks = (float)(log2e / (2.0 * (double)fp->sigma_space_px * fp->sigma_space_px));
   float kr = (float)(log2e / (2.0 * (double)fp->sigma_range_mm * fp->sigma_range_mm));
   if (fp->radius_px == -1) {
-    dim3 blk(32, 8);
+    dim3 blk(kTileX, kTileY);
     dim3 grid((cam->width + 31) / 32, (cam->height + 7) / 8);
     k_depth_raw<<<grid, blk, 0, s>>>(d_depth, pitch, cam->width, cam->height, cam->min_depth_mm,
                                      cam->max_depth_mm, (float *)(base + lay.depth_offset[0]));
   } else {
-    dim3 grid((cam->width + kTileX - 1) / kTileX, (cam->height + kTileY - 1) / kTileY);
-    size_t smem = (size_t)(kTileX + 2 * R) * (kTileY + 2 * R) * sizeof(float);
     float *o = (float *)(base + lay.depth_offset[0]);
     const int W = cam->width, H = cam->height;
     const float dmn = cam->min_depth_mm, dmx = cam->max_depth_mm;
-#define OF_BILATERAL_CASE(RR)                                                           \
-  case RR: {                                                                            \
-    size_t dyn_ = 0;                                                                    \
-    const cudaError_t fe_ = filter_footprint(k_bilateral_r<RR>, &dyn_);                 \
-    if (fe_ != cudaSuccess) return of_set_cuda_error(fe_);                              \
-    k_bilateral_r<RR><<<grid, kTileX * kTileY, dyn_, s>>>(d_depth, pitch, W, H, dmn, dmx, \
-                                                           ks, kr, o);                  \
-  } break;
+#define OF_BILATERAL_CASE(RR)                                                             \
+  case RR:                                                                              \
+    st = launch_bilateral<RR>(d_depth, pitch, W, H, dmn, dmx, ks, kr, o, s, captured);  \
+    if (st != OF_OK) return st;                                                         \
+    break;
     switch (R) {
+      OF_BILATERAL_CASE(1)
+      OF_BILATERAL_CASE(2)
       OF_BILATERAL_CASE(3)
       OF_BILATERAL_CASE(4)
       OF_BILATERAL_CASE(5)
@@ -517,30 +614,30 @@ extern "C" of_status_t of_preprocess(const of_camera_t *cam, const of_filter_par
       OF_BILATERAL_CASE(8)
       OF_BILATERAL_CASE(9)
       OF_BILATERAL_CASE(10)
+      OF_BILATERAL_CASE(11)
       OF_BILATERAL_CASE(12)
+      OF_BILATERAL_CASE(13)
+      OF_BILATERAL_CASE(14)
+      OF_BILATERAL_CASE(15)
+      OF_BILATERAL_CASE(16)
       default:
-        k_bilateral<<<grid, kTileX * kTileY, smem, s>>>(d_depth, pitch, W, H, dmn, dmx, R, ks, kr,
-                                                        o);
+        return OF_ERR_INVALID_ARGUMENT;  // (R is 1 .. kMaxRadius here)
     }
 #undef OF_BILATERAL_CASE
   }
-  float guard = 3.0f * fp->sigma_range_mm;
-  for (int l = 1; l < fp->levels; ++l) {
-    dim3 blk(32, 8);
-    dim3 grid((lay.width[l] + 31) / 32, (lay.height[l] + 7) / 8);
-    k_pyr_down<<<grid, blk, 0, s>>>((const float *)(base + lay.depth_offset[l - 1]),
-                                    lay.width[l - 1], lay.height[l - 1],
-                                    (float *)(base + lay.depth_offset[l]), lay.width[l],
-                                    lay.height[l], guard);
-  }
-  for (int l = 0; l < fp->levels; ++l) {
-    of_camera_t c = camera_level(*cam, l);
-    dim3 blk(32, 8);
-    dim3 grid((c.width + 31) / 32, (c.height + 7) / 8);
-    k_vertex_normal<<<grid, blk, 0, s>>>((const float *)(base + lay.depth_offset[l]), c.width,
-                                         c.height, c.cx, c.cy, (float)(1.0 / (double)c.fx),
-                                         (float)(1.0 / (double)c.fy),
-                                         (float4 *)(base + lay.points_offset[l]));
-  }
+  // outside a capture the pyramid is launched programmatically: its blocks
+  // start as the filter's last ones run (a captured graph launches its nodes
+  // back to back already)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((cam->width + kPyrTile - 1) / kPyrTile, (cam->height + kPyrTile - 1) / kPyrTile);
+  cfg.blockDim = dim3(kPyrThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = captured ? 0 : 1;
+  OF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pyramid, pyramid_maps(*cam, lay, fp->levels, base),
+                                 3.0f * fp->sigma_range_mm));
   return of_launch_status();
 }
