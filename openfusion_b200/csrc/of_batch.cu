@@ -84,6 +84,70 @@ void release(of_batch *b) {
   delete b;
 }
 
+// Device frames into the streams' depth buffers, one launch for up to
+// kCopyFrames of them (a copy each took 2 us a stream, one after another): 16
+// bytes a thread where the source allows it, else pixel by pixel.
+constexpr int kCopyFrames = 128, kCopyThreads = 256, kCopyVecs = 4;
+struct FrameCopies {
+  const uint16_t *src[kCopyFrames];
+  uint16_t *dst[kCopyFrames];
+  int pixels[kCopyFrames];
+};
+static_assert(sizeof(FrameCopies) <= 4000, "kernel parameters");
+__global__ void __launch_bounds__(kCopyThreads) k_copy_frames(FrameCopies C) {
+  const int f = blockIdx.y, px = C.pixels[f];
+  const uint16_t *src = C.src[f];
+  uint16_t *dst = C.dst[f];
+  const int first = blockIdx.x * kCopyThreads * kCopyVecs * 8;
+  const bool vec = ((uintptr_t)src & 15u) == 0;
+#pragma unroll
+  for (int k = 0; k < kCopyVecs; ++k) {
+    const int p = first + (k * kCopyThreads + (int)threadIdx.x) * 8;
+    if (vec && p + 8 <= px) {
+      *reinterpret_cast<uint4 *>(dst + p) = __ldg(reinterpret_cast<const uint4 *>(src + p));
+    } else {
+      for (int i = p; i < min(p + 8, px); ++i) dst[i] = src[i];
+    }
+  }
+}
+
+// Copies every stream's frame: one launch a group for frames in this device's
+// own memory, a copy for any other.
+of_status_t copy_frames(of_batch *b, const uint16_t *const *depth, bool host, int cur, cudaStream_t s) {
+  int dev = 0;
+  OF_CUDA_TRY(cudaGetDevice(&dev));
+  FrameCopies C;
+  int m = 0, most = 0;
+  auto flush = [&]() {
+    if (m == 0) return cudaSuccess;
+    const int per = kCopyThreads * kCopyVecs * 8;
+    k_copy_frames<<<dim3((most + per - 1) / per, m), kCopyThreads, 0, s>>>(C);
+    m = most = 0;
+    return cudaGetLastError();
+  };
+  for (int i = 0; i < b->desc.count; ++i) {
+    const int px = b->bs[i].cam.width * b->bs[i].cam.height;
+    uint16_t *dst = (uint16_t *)b->bs[i].depth[cur];
+    if (depth[i] == dst) continue;
+    cudaPointerAttributes a = {};
+    const bool own = !host && cudaPointerGetAttributes(&a, depth[i]) == cudaSuccess &&
+                     a.type == cudaMemoryTypeDevice && a.device == dev;
+    if (!own) {
+      if (!host) cudaGetLastError();  // (an unknown pointer: the copy reports it)
+      OF_CUDA_TRY(cudaMemcpyAsync(dst, depth[i], (size_t)px * sizeof(uint16_t),
+                                  host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
+      continue;
+    }
+    C.src[m] = depth[i];
+    C.dst[m] = dst;
+    C.pixels[m++] = px;
+    most = px > most ? px : most;
+    if (m == kCopyFrames) OF_CUDA_TRY(flush());
+  }
+  OF_CUDA_TRY(flush());
+  return OF_OK;
+}
+
 // fuse every stream's frame in depth[parity] at its pose, raycast the models
 of_status_t enqueue_fuse(of_batch *b, int parity, cudaStream_t s, bool timed) {
   if (timed) OF_CUDA_TRY(cudaEventRecord(b->ev_t[0], s));
@@ -222,8 +286,9 @@ extern "C" of_status_t of_batch_create(const of_batch_desc_t *desc, of_batch_t *
   for (int i = 0; i < 5 && e == cudaSuccess; ++i) e = cudaEventCreate(&b->ev_t[i]);
   if (e != cudaSuccess) { release(b); return of_set_cuda_error(e); }
   // one arena: per stream volume, lambda table, integration scratch, frame
-  // and model pyramids, two depth buffers, pose, ICP statistics
-  struct Off { size_t vol, lam, scratch, frame, model, depth0, depth1, pose, stats; };
+  // and model pyramids, two depth buffers; then every stream's pose and every
+  // stream's ICP statistics, each in a row (of_batch_poses copies them whole)
+  struct Off { size_t vol, lam, scratch, frame, model, depth0, depth1; };
   std::vector<Off> off(n);
   size_t total = 0;
   for (int i = 0; i < n; ++i) {
@@ -244,9 +309,11 @@ extern "C" of_status_t of_batch_create(const of_batch_desc_t *desc, of_batch_t *
     o.model = total; total = a256(total + lay.total_bytes);
     o.depth0 = total; total = a256(total + px);
     o.depth1 = total; total = a256(total + px);
-    o.pose = total; total = a256(total + 16 * sizeof(double));
-    o.stats = total; total = a256(total + sizeof(of_icp_stats_t));
   }
+  const size_t poses_off = total;
+  total = a256(total + (size_t)n * 16 * sizeof(double));
+  const size_t stats_off = total;
+  total = a256(total + (size_t)n * sizeof(of_icp_stats_t));
   e = cudaMalloc(&b->arena, total);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -269,8 +336,8 @@ extern "C" of_status_t of_batch_create(const of_batch_desc_t *desc, of_batch_t *
     B.model = base + off[i].model;
     B.depth[0] = (const uint16_t *)(base + off[i].depth0);
     B.depth[1] = (const uint16_t *)(base + off[i].depth1);
-    B.pose = (double *)(base + off[i].pose);
-    B.stats = (of_icp_stats_t *)(base + off[i].stats);
+    B.pose = (double *)(base + poses_off) + 16 * (size_t)i;
+    B.stats = (of_icp_stats_t *)(base + stats_off) + i;
     st = of_volume_reset(&S.volume, B.volume, s);
     if (st == OF_OK) st = of_lambda_table(&S.camera, (float *)B.lambda, s);
     of_pyramid_layout_t lay;
@@ -331,13 +398,8 @@ extern "C" of_status_t of_batch_process(of_batch_t b, const uint16_t *const *dep
     if (!depth[i]) return OF_ERR_INVALID_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
   const int cur = (int)(b->frames & 1);
-  for (int i = 0; i < n; ++i) {
-    const size_t bytes = (size_t)b->bs[i].cam.width * b->bs[i].cam.height * sizeof(uint16_t);
-    uint16_t *dst = (uint16_t *)b->bs[i].depth[cur];
-    if (depth[i] != dst)
-      OF_CUDA_TRY(cudaMemcpyAsync(dst, depth[i], bytes,
-                                  depth_is_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
-  }
+  const of_status_t sc = copy_frames(b, depth, depth_is_host != 0, cur, s);
+  if (sc != OF_OK) return sc;
   if (b->frames > 0) {
     const bool fuse = !b->last_fused;
     if (b->tuned && b->desc.use_graph && fuse) {
@@ -371,13 +433,13 @@ extern "C" of_status_t of_batch_poses(of_batch_t b, double *poses, of_icp_stats_
                                       of_stream_t stream) {
   if (!b || !poses) return OF_ERR_INVALID_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
-  for (int i = 0; i < b->desc.count; ++i) {
-    OF_CUDA_TRY(cudaMemcpyAsync(poses + 16 * (size_t)i, b->bs[i].pose, 16 * sizeof(double),
+  // (one copy each: a copy a stream, each waited for when the caller's memory
+  // is pageable, took 105 us for 16 streams)
+  const size_t n = (size_t)b->desc.count;
+  OF_CUDA_TRY(cudaMemcpyAsync(poses, b->bs[0].pose, n * 16 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  if (stats)
+    OF_CUDA_TRY(cudaMemcpyAsync(stats, b->bs[0].stats, n * sizeof(of_icp_stats_t),
                                 cudaMemcpyDeviceToHost, s));
-    if (stats)
-      OF_CUDA_TRY(cudaMemcpyAsync(stats + i, b->bs[i].stats, sizeof(of_icp_stats_t),
-                                  cudaMemcpyDeviceToHost, s));
-  }
   return OF_OK;
 }
 

@@ -34,3 +34,43 @@ def test_both_cluster_sizes_give_the_same_poses(of, cuda, w, h):
             assert all(s.status == 0 for s in sp) and (k == 0 or all(s.inliers > 100 for s in sp))
     few.close()
     many.close()
+
+
+def test_frames_from_anywhere_are_the_same(of, cuda):
+    """Device frames at 16-byte boundaries, at odd pixels, and host frames, of
+    more streams than one copy launch takes and of sizes off its 8 pixels."""
+    import torch
+    base = dataclasses.replace(of.CONFIGS["c1"], resolution=32, max_depth_mm=4000.0)
+    cfgs = [dataclasses.replace(base, width=w, height=h, cx=w / 2, cy=h / 2)
+            for w, h in ((17, 13), (24, 18), (40, 31))]
+    cfgs = [cfgs[i % 3] for i in range(131)]
+    rng = np.random.default_rng(0)
+    host = [[torch.from_numpy(rng.integers(400, 3000, (c.height, c.width)).astype(np.int16)) for c in cfgs]
+            for _ in range(2)]
+
+    def shifted(t):
+        buf = torch.zeros(t.numel() + 1, dtype=torch.int16, device=cuda)
+        buf[1:] = t.reshape(-1).to(cuda)
+        return buf[1:]
+
+    out = []
+    for place in (lambda t: t.to(cuda), shifted, lambda t: t):
+        b = of.Batch(cfgs, [np.eye(4)] * len(cfgs), use_graph=False)
+        frames = []
+        for k in range(2):
+            depth = [place(t) for t in host[k]]
+            b.process(depth)
+            torch.cuda.synchronize()
+            for i, c in enumerate(cfgs):
+                got = torch.as_tensor(_Words(b.buffers(i).depth, c.width * c.height), device=cuda)
+                frames.append(got.cpu())
+                assert torch.equal(frames[-1], host[k][i].reshape(-1))
+        out.append(b.poses())
+        b.close()
+    assert np.array_equal(out[0], out[1], equal_nan=True) and np.array_equal(out[0], out[2], equal_nan=True)
+
+
+class _Words:
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": "<i2", "data": (int(ptr), False),
+                                         "version": 3}
