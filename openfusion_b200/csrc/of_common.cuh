@@ -121,6 +121,37 @@ __device__ inline void pose_to_rigid(const double *P, Rigid *c2w, Rigid *w2c) {
   }
 }
 
+// ---------------------------------------------------------- paired FP32 --
+
+// Two FP32 values an instruction (each half rounded as the scalar form rounds).
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 z, x, y; "
+      "mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 z, x, y; "
+      "mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{.reg .b64 x, y, z, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; "
+      "fma.rn.f32x2 w, x, y, z; mov.b64 {%0, %1}, w;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+// a - b
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  return fma2(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+
 // ------------------------------------------------- float-pair arithmetic --
 // Error-free transformations (Knuth two-sum, fma two-product) used where an
 // FP32 result must match an FP64 oracle to better than one int16 tsdf step.
@@ -156,6 +187,41 @@ __device__ __forceinline__ float2 df_sqrt(float2 a) {
   const float r = pos ? a.x * y : 0.f;
   const float e = __fadd_rn(__fmaf_rn(-r, r, a.x), a.y);
   return make_float2(r, pos ? e * (0.5f * y) : 0.f);
+}
+
+// The same on two float pairs at once (hi and lo parts of both in a float2
+// each): every step rounds as the scalar form's.
+struct DfPair {
+  float2 hi, lo;
+};
+__device__ __forceinline__ DfPair two_sum2(float2 a, float2 b) {
+  const float2 s = add2(a, b);
+  const float2 bb = sub2(s, a);
+  return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
+}
+__device__ __forceinline__ DfPair two_prod2(float2 a, float2 b) {
+  const float2 p = mul2(a, b);
+  return {p, fma2(a, b, mul2(p, make_float2(-1.f, -1.f)))};
+}
+__device__ __forceinline__ DfPair df_sq2(DfPair x) {
+  DfPair p = two_prod2(x.hi, x.hi);
+  p.lo = fma2(add2(x.hi, x.hi), x.lo, p.lo);
+  return p;
+}
+__device__ __forceinline__ DfPair df_add2(DfPair a, DfPair b) {
+  const DfPair s = two_sum2(a.hi, b.hi);
+  return two_sum2(s.hi, add2(s.lo, add2(a.lo, b.lo)));
+}
+// (a zero or subnormal high part has root 0 here, below any use's precision)
+__device__ __forceinline__ DfPair df_sqrt2(DfPair a) {
+  float2 y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(a.hi.x));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(a.hi.y));
+  y.x = a.hi.x >= 1.17549435e-38f ? y.x : 0.f;
+  y.y = a.hi.y >= 1.17549435e-38f ? y.y : 0.f;
+  const float2 r = mul2(a.hi, y);
+  const float2 e = add2(fma2(mul2(r, make_float2(-1.f, -1.f)), r, a.hi), a.lo);
+  return {r, mul2(e, mul2(dup2(0.5f), y))};
 }
 
 // ------------------------------------------------------------------ voxels --
