@@ -759,10 +759,15 @@ __device__ __forceinline__ void integrate_list_block(uint32_t *__restrict__ vol,
   for (unsigned c = bx; c < nchunks; buf ^= 1) {
     unsigned nxt = 0;
     if (threadIdx.x == 0) nxt = gx + atomicAdd(next, 1u);
-    for (unsigned k = warp >> 2; k < kChunkBricks; k += 2) {
-      const unsigned e = c + k * nchunks;
-      if (e >= n) break;
-      const uint4 en = __ldg(list + e);
+    // the warp's entries of the chunk, a lane each, in one request
+    constexpr unsigned kMine = kChunkBricks / 2;
+    uint4 mine = make_uint4(0u, 0u, 0u, 0u);
+    const unsigned e0 = c + (warp >> 2) * nchunks;
+    if ((unsigned)lane < kMine && e0 + 2u * lane * nchunks < n) mine = __ldg(list + e0 + 2u * lane * nchunks);
+    for (unsigned k = 0; k < kMine; ++k) {
+      if (e0 + 2u * k * nchunks >= n) break;
+      const uint4 en = make_uint4(__shfl_sync(0xffffffffu, mine.x, k), __shfl_sync(0xffffffffu, mine.y, k),
+                                  __shfl_sync(0xffffffffu, mine.z, k), __shfl_sync(0xffffffffu, mine.w, k));
       const int bx = (int)(en.x & 0xffu), by = (int)((en.x >> 8) & 0xffu);
       const int bz = (int)((en.x >> 16) & 0xffu), mode = (int)((en.x >> 24) & 3u);
       const int sat_old = (int)((en.x >> 26) & 0xfu);
