@@ -38,7 +38,12 @@ constexpr int kIcpMaxBlocks = 2 * kSmCount;
 constexpr int kVals = 29;  // 21 + 6 + residual^2 + inliers
 constexpr float kEps = 1e-6f;  // _EPSILON_ (Constants.h:14)
 
-constexpr int kFusedThreads = 1024;
+// A block's sums run as kFusedChains chains (a chain: every kFusedChains-th
+// cached point, then a lane of the remaining chunks), 32 chains a warp sum; a
+// thread carries two of them, kFusedThreads apart.
+constexpr int kFusedThreads = 512;
+constexpr int kFusedChains = 1024;
+constexpr int kChainWarps = kFusedChains / 32;
 constexpr int kFusedMaxBlocks = 2 * kSmCount;
 // model points a block of the fused kernel keeps in shared memory (192 KiB)
 constexpr int kMaxCachePts = 6144;
@@ -320,9 +325,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_gpu(unsigned *p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long ld_relaxed_gpu(const unsigned long long *p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -399,90 +401,111 @@ __device__ __forceinline__ void sincos_small(double x, double *s, double *c) {
   *c = fma(-x2, pc, 1.0);
 }
 
-// Warp-parallel FP64 solve of the 6x6 normal equations (21 upper entries and
-// 6 right-hand sides in tot[0..26], inliers in tot[28]) and the SE(3) update
-// of P (row-major 4x4, shared memory); all 32 lanes of one warp call it.
-// Lane i < 6 holds row i of [H | g] and the rows are eliminated in order
-// (Gaussian elimination without pivoting, which on the symmetric system is the
-// LDL^T factorisation: its pivots d_j equal the squared Cholesky pivots, so
-// the singularity rule is the Cholesky solve's: a pivot not above 1e-12 x the
-// largest diagonal entry, a non-finite pivot, or fewer than 6 inliers). Back
-// substitution by one shuffle per unknown, rotation part negated
-// (ICP.cpp:162-168), dT = [Rz(g) Ry(b) Rx(a) | t] (ICP.cu:274-290) and
-// P <- dT P with one entry per lane. Returns the warp-uniform success flag;
-// *minpiv gets min d_j / max H_ii, *inc_rot / *inc_trans the largest
-// rotation (rad) / translation (mm) component of the increment. With c2w /
-// w2c given, the lanes also write the FP32 rigid transforms of the new pose
-// (pose_to_rigid's values) on success.
+// FP64 solve of the 6x6 normal equations (21 upper entries and 6 right-hand
+// sides in tot[0..26], inliers in tot[28]; tot holds 32 values) and the SE(3)
+// update of P (row-major 4x4, shared memory); all 32 lanes of one warp call it,
+// `sys` is a shared array of 32. The rows are eliminated in order (Gaussian
+// elimination without pivoting, which on the symmetric system is the LDL^T
+// factorisation: its pivots d_j equal the squared Cholesky pivots, so the
+// singularity rule is the Cholesky solve's: a pivot not above 1e-12 x the
+// largest diagonal entry, a non-finite pivot, or fewer than 6 inliers).
+// Rotation part negated (ICP.cpp:162-168), dT = [Rz(g) Ry(b) Rx(a) | t]
+// (ICP.cu:274-290) and P <- dT P with one entry per lane. Returns the
+// warp-uniform success flag. With c2w / w2c given, the lanes also write the
+// FP32 rigid transforms of the new pose (pose_to_rigid's values) on success.
+// It is a chain of dependent FP64 instructions that every block waits for in
+// every iteration, so all lanes hold the whole system (a row a lane needs an
+// exchange at each pivot and unknown) and what only the frame's end reads is
+// left to it: with the exchange
+// of the rows' slots requested together and two chains a thread, ICP of a
+// 640x480 frame (19 iterations) 136.5 -> 113.6 us.
 __device__ __forceinline__ double shfl_d(double v, int src) {
   return __shfl_sync(0xffffffffu, v, src);
 }
 __device__ __forceinline__ int upper_index(int i, int j) {  // i <= j
   return i * 6 - i * (i - 1) / 2 + (j - i);
 }
-__device__ bool warp_solve_update(const float *tot, double *P, double *minpiv, float *inc_rot,
-                                  float *inc_trans, Rigid *c2w = nullptr, Rigid *w2c = nullptr) {
+struct SolveInfo {
+  double dmin, dmax;          // smallest pivot, largest diagonal entry
+  float inc_rot, inc_trans;   // the increment's largest components
+};
+// smallest pivot over the largest diagonal entry (not positive when singular)
+__device__ __forceinline__ double min_pivot(const SolveInfo &o, bool ok) {
+  return ok ? o.dmin / o.dmax : fmin(o.dmin / o.dmax, 0.0);
+}
+__device__ bool warp_solve_update(const float *tot, double *sys, double *P, SolveInfo *info,
+                                  Rigid *c2w = nullptr, Rigid *w2c = nullptr) {
   const int lane = threadIdx.x & 31;
-  const int row = lane < 6 ? lane : 5;  // lanes 6.. shadow row 5
-  double a[7];
+  sys[lane] = (double)tot[lane];  // (28 used: a lane converts one)
+  __syncwarp();
+  double a[6][7], r[6], x[6];
 #pragma unroll
-  for (int k = 0; k < 6; ++k)
-    a[k] = (double)tot[row <= k ? upper_index(row, k) : upper_index(k, row)];
-  a[6] = (double)tot[21 + row];
-  double dmax = 0.0;
+  for (int i = 0; i < 6; ++i) {
 #pragma unroll
-  for (int i = 0; i < 6; ++i) dmax = fmax(dmax, (double)tot[upper_index(i, i)]);
+    for (int k = 0; k < 6; ++k) a[i][k] = sys[i <= k ? upper_index(i, k) : upper_index(k, i)];
+    a[i][6] = sys[21 + i];
+  }
+  const double dmax = fmax(fmax(fmax(fmax(0.0, a[0][0]), a[1][1]), fmax(a[2][2], a[3][3])),
+                           fmax(a[4][4], a[5][5]));
   bool ok = tot[28] >= 6.f && dmax > 0.0 && isfinite(dmax);
   const double thr = 1e-12 * dmax;
-  double dmin = 1e300, rmine = 0.0;
+  // every lane eliminates the whole system: a pivot's chain is its reciprocal,
+  // a product and an fma, with no exchange between lanes
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    double pj[7];
+    r[j] = recip_pos(a[j][j]);
+    ok = ok && (a[j][j] > thr) && isfinite(a[j][j]);
 #pragma unroll
-    for (int k = j; k < 7; ++k) pj[k] = shfl_d(a[k], j);
-    const double dj = pj[j];
-    dmin = fmin(dmin, dj);
-    ok = ok && (dj > thr) && isfinite(dj);
-    const double rj = recip_pos(fmax(dj, 1e-300));
-    if (row == j) rmine = rj;
-    if (row > j) {
-      const double f = a[j] * rj;
+    for (int i = j + 1; i < 6; ++i) {
+      const double f = a[i][j] * r[j];
 #pragma unroll
-      for (int k = j + 1; k < 7; ++k) a[k] = fma(-f, pj[k], a[k]);
+      for (int k = j + 1; k < 7; ++k) a[i][k] = fma(-f, a[j][k], a[i][k]);
     }
   }
-  *minpiv = ok ? dmin / dmax : fmin(dmin / dmax, 0.0);
+  info->dmin = fmin(fmin(fmin(a[0][0], a[1][1]), fmin(a[2][2], a[3][3])), fmin(a[4][4], a[5][5]));
+  info->dmax = dmax;
   if (!ok) return false;
-  double x[6];
 #pragma unroll
   for (int i = 5; i >= 0; --i) {
-    x[i] = shfl_d(a[6] * rmine, i);
-    if (row < i) a[6] = fma(-a[i], x[i], a[6]);
+    x[i] = a[i][6] * r[i];
+#pragma unroll
+    for (int k = 0; k < i; ++k) a[k][6] = fma(-a[k][i], x[i], a[k][6]);
   }
-  *inc_rot = (float)fmax(fabs(x[0]), fmax(fabs(x[1]), fabs(x[2])));
-  *inc_trans = (float)fmax(fabs(x[3]), fmax(fabs(x[4]), fabs(x[5])));
-  double sv = 0.0, cv = 1.0;
-  if (lane < 3) sincos_small(-x[lane], &sv, &cv);
-  const double sa = shfl_d(sv, 0), ca = shfl_d(cv, 0);
-  const double sb = shfl_d(sv, 1), cb = shfl_d(cv, 1);
-  const double sg = shfl_d(sv, 2), cg = shfl_d(cv, 2);
+  double sa, ca, sb, cb, sg, cg;
+  sincos_small(-x[0], &sa, &ca);
+  sincos_small(-x[1], &sb, &cb);
+  sincos_small(-x[2], &sg, &cg);
   // lane l < 12 forms entry (l / 4, l % 4) of dT P; row 3 stays 0 0 0 1
-  const int r = (lane >> 2) % 3, c = lane & 3;
+  // (rounded products and sums: no fma, whatever the code around them)
+  const int q = (lane >> 2) % 3, c = lane & 3;
   double D0, D1, D2, D3;
-  if (r == 0) { D0 = cg * cb; D1 = -sg * ca + cg * sb * sa; D2 = sg * sa + cg * sb * ca; D3 = x[3]; }
-  else if (r == 1) { D0 = sg * cb; D1 = cg * ca + sg * sb * sa; D2 = -cg * sa + sg * sb * ca; D3 = x[4]; }
-  else { D0 = -sb; D1 = cb * sa; D2 = cb * ca; D3 = x[5]; }
+  if (q == 0) {
+    D0 = cg * cb;
+    D1 = __dadd_rn(__dmul_rn(-sg, ca), __dmul_rn(cg * sb, sa));
+    D2 = __dadd_rn(__dmul_rn(sg, sa), __dmul_rn(cg * sb, ca));
+    D3 = x[3];
+  } else if (q == 1) {
+    D0 = sg * cb;
+    D1 = __dadd_rn(__dmul_rn(cg, ca), __dmul_rn(sg * sb, sa));
+    D2 = __dadd_rn(__dmul_rn(-cg, sa), __dmul_rn(sg * sb, ca));
+    D3 = x[4];
+  } else {
+    D0 = -sb;
+    D1 = cb * sa;
+    D2 = cb * ca;
+    D3 = x[5];
+  }
   const double v = fma(D0, P[c], fma(D1, P[4 + c], fma(D2, P[8 + c], D3 * P[12 + c])));
   __syncwarp();
   if (lane < 12) P[lane] = v;
   if (c2w) {
-    // entry (r, c) of the new pose is v on lane 4 r + c (lanes 0..11)
+    // entry (q, c) of the new pose is v on lane 4 q + c (lanes 0..11)
     if (lane < 12) {
       if (c < 3) {
-        c2w->r[3 * r + c] = (float)v;
-        w2c->r[3 * c + r] = (float)v;
+        c2w->r[3 * q + c] = (float)v;
+        w2c->r[3 * c + q] = (float)v;
       } else {
-        c2w->t[r] = (float)v;
+        c2w->t[q] = (float)v;
       }
     }
     // w2c.t[i] = -(column i of R) . t, lane i < 3
@@ -497,6 +520,8 @@ __device__ bool warp_solve_update(const float *tot, double *P, double *minpiv, f
       w2c->t[lane] = (float)acc;
     }
   }
+  info->inc_rot = (float)fmax(fabs(x[0]), fmax(fabs(x[1]), fabs(x[2])));
+  info->inc_trans = (float)fmax(fabs(x[3]), fmax(fabs(x[4]), fabs(x[5])));
   __syncwarp();
   return true;
 }
@@ -546,6 +571,95 @@ __device__ __forceinline__ void try_row(float *acc, const Rigid &c2w, float4 s, 
   add_row(acc, s, ns, d);
 }
 
+// A point of a pyramid (vertex, normal): one 32-byte load where the pyramid
+// starts at a 32-byte boundary (the trackers' own do), else two of 16.
+struct MapPoint {
+  float4 v, n;
+};
+__device__ __forceinline__ MapPoint ld_point(const float4 *p) {
+  MapPoint m;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(m.v.x), "=f"(m.v.y), "=f"(m.v.z), "=f"(m.v.w), "=f"(m.n.x), "=f"(m.n.y), "=f"(m.n.z),
+        "=f"(m.n.w)
+      : "l"(p));
+  return m;
+}
+template <bool WIDE>
+__device__ __forceinline__ MapPoint load_point(const float4 *p) {
+  if (WIDE) return ld_point(p);
+  return {__ldg(p), __ldg(p + 1)};
+}
+
+// 1 / z rounded to nearest for |z| in [2^-126, 2^126), without a branch: the
+// approximate reciprocal, a Newton step, and Markstein's final step (IBM
+// Journal of R&D 34, 1990), which rounds correctly from an approximation that
+// is right to within an ulp. Equal to __frcp_rn for every mantissa, sign and
+// exponent of that range (checked on B200 over all of them).
+__device__ __forceinline__ float recip_rn(float z) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(z));
+  y = __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
+  return __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
+}
+// associate() without a branch: the frame pixel (0 if none), and whether the
+// point projects into the frame.
+__device__ __forceinline__ int associate_flat(const Rigid &w2c, const Cam &cam, float3 s, bool &seen) {
+  const float3 sc = apply(w2c, s);
+  const float rz = recip_rn(sc.z);
+  const int pu = __float2int_rd(fmaf(cam.fx * sc.x, rz, cam.cx) + 0.5f);
+  const int pv = __float2int_rd(fmaf(cam.fy * sc.y, rz, cam.cy) + 0.5f);
+  seen = seen && !(sc.z >= -kEps) && (unsigned)pu < (unsigned)cam.w && (unsigned)pv < (unsigned)cam.h;
+  return seen ? pv * cam.w + pu : 0;
+}
+
+// A model point, the frame point at its pixel, and whether it has one.
+struct BatchPoint {
+  float3 s, ns;
+  MapPoint f;
+  bool seen;
+};
+__device__ __forceinline__ BatchPoint batch_frame(const MapPoint &m, bool live, const Rigid &w2c,
+                                                  const Cam &cam, const float4 *__restrict__ frame) {
+  BatchPoint b;
+  b.s = make_float3(m.v.x, m.v.y, m.v.z);
+  b.ns = make_float3(m.n.x, m.n.y, m.n.z);
+  b.seen = live && m.v.w != 0.f && m.n.w != 0.f;
+  const int q = associate_flat(w2c, cam, b.s, b.seen);
+  b.f = ld_point(frame + 2 * q);
+  return b;
+}
+// The point's row a[0..5], b = a[6] and inlier count a[7] (try_row's tests and
+// arithmetic); zeros when it is no inlier.
+__device__ __forceinline__ void batch_row(float (&a)[8], const Rigid &c2w, const BatchPoint &p,
+                                          float dist2, float nthr) {
+  const float3 s = p.s, ns = p.ns;
+  const float3 d = apply(c2w, make_float3(p.f.v.x, p.f.v.y, p.f.v.z));
+  const float3 nd = rotate(c2w, make_float3(p.f.n.x, p.f.n.y, p.f.n.z));
+  const float ex = d.x - s.x, ey = d.y - s.y, ez = d.z - s.z;
+  const float dn = nd.x * ns.x + nd.y * ns.y + nd.z * ns.z;
+  const bool ok = p.seen && p.f.v.w != 0.f && p.f.n.w != 0.f &&
+                  fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < dist2 && dn > nthr && dn < 1.f + kEps;
+  a[0] = ok ? ns.y * d.z - ns.z * d.y : 0.f;
+  a[1] = ok ? ns.z * d.x - ns.x * d.z : 0.f;
+  a[2] = ok ? ns.x * d.y - ns.y * d.x : 0.f;
+  a[3] = ok ? ns.x : 0.f;
+  a[4] = ok ? ns.y : 0.f;
+  a[5] = ok ? ns.z : 0.f;
+  a[6] = ok ? -(ns.x * ex + ns.y * ey + ns.z * ez) : 0.f;
+  a[7] = ok ? 1.f : 0.f;
+}
+__device__ __forceinline__ void batch_add(float *acc, const float (&a)[8]) {
+  int k = 0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int j = i; j < 6; ++j) { acc[k] = fmaf(a[i], a[j], acc[k]); ++k; }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) acc[21 + i] = fmaf(a[i], a[6], acc[21 + i]);
+  acc[27] = fmaf(a[6], a[6], acc[27]);
+  acc[28] += a[7];
+}
+
 // Judge of a warm-started ICP result P (warm start W): kept when the last
 // iteration's RMS point-to-plane residual, its inlier fraction among the
 // examined model points, and its rotation / translation away from W are all
@@ -570,23 +684,29 @@ __device__ __forceinline__ bool judge_keep(const IcpPlan &plan, const double *W,
 // start of a level it copies its chunks' valid model points (vertex, normal)
 // into shared memory in chunk order, up to the dynamic shared-memory capacity
 // (the rest is read from global memory at every iteration). Per
-// iteration: every block associates its points two at a time (both frame
-// gathers in flight together), accumulates the rows (tree sums), writes 29
-// partials, meets the others at one grid barrier, then reduces all blocks'
-// partials in the same fixed order and one warp solves the 6x6 system, so
-// every block holds the same new pose without a second barrier. Partials
+// iteration: every thread associates up to four of the block's points (their
+// frame gathers in flight together, no branch between them), accumulates the
+// rows of its two chains (tree sums), the block writes 29 partials, meets the
+// others at one grid barrier, then reduces all blocks' partials in the same
+// fixed order and one warp solves the 6x6 system, so every block holds the same
+// new pose without a second barrier. Bound by latency: the slowest block's
+// rows, the rows' way through L2, the solve. (512 threads with two chains each
+// rather than 1024 with one: the branch-free points want 128 registers.) Partials
 // alternate between two buffers: a block can only overwrite buffer i%2 after
 // the barrier of iteration i+1, which every block reaches only after reading it.
+template <bool WIDE, int ROWS>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     k_icp_fused(IcpPlan plan, double *pose, IcpWorkspace *ws, of_icp_stats_t *stats) {
   extern __shared__ float4 s_pts[];  // 2 per cached model point
   __shared__ double s_pose[16];
   __shared__ Rigid s_c2w, s_w2c;
-  __shared__ float s_red[kFusedThreads / 32][32];
+  __shared__ float s_red[kChainWarps][32];
   __shared__ float s_tot[32];
+  __shared__ double s_sys[32];
   __shared__ int s_chunk_off[kMaxCachePts / 32];  // per cached chunk: its valid points, then their offset
-  __shared__ int s_stop, s_inl, s_its, s_err, s_npts, s_conv, s_warm, s_examined;
-  __shared__ double s_res, s_piv;
+  __shared__ int s_stop, s_err, s_npts, s_conv, s_warm;
+  __shared__ SolveInfo s_info;  // of the last solve (its sums stay in s_tot)
+  __shared__ bool s_solved;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kWarps = kFusedThreads / 32;
   // pass 0 starts from the warm start when this frame has one, else from the
@@ -598,11 +718,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   if (threadIdx.x < 16)
     s_pose[threadIdx.x] = warm ? ws->warm_pose[threadIdx.x] : ws->pose_init[threadIdx.x];
   if (threadIdx.x == 0) {
-    s_stop = 0; s_err = 0; s_its = 0; s_inl = 0; s_res = 0.0; s_piv = 0.0; s_examined = 0;
+    s_stop = 0; s_err = 0;
     s_warm = warm ? 1 : 0;
   }
   __syncthreads();  // every thread reads the flags and the pose below
   if (threadIdx.x == 0) pose_to_rigid(s_pose, &s_c2w, &s_w2c);
+  if (threadIdx.x < 32) s_tot[threadIdx.x] = 0.f;
   // the fault-injection hook holds every exchange for an arrival that never
   // comes
   const bool hold = ws->hold_barrier > 0;
@@ -680,78 +801,96 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       __syncthreads();
       const int n = s_npts;
       for (int it = 0; it < L.iters; ++it) {
-        float acc[kVals];
-        float examined = 0.f;  // model points that project into the frame
+        // the frame points of the thread's first four cached points (two of
+        // each chain), requested before any is used
+        BatchPoint pt[4];
 #pragma unroll
-        for (int v = 0; v < kVals; ++v) acc[v] = 0.f;
-        // cached points, two per step
-        for (int i = threadIdx.x; i < n; i += 2 * kFusedThreads) {
-          const int j = i + kFusedThreads;
-          const int qA = associate(s_w2c, L.cam, s_pts[2 * i]);
-          const int qB = j < n ? associate(s_w2c, L.cam, s_pts[2 * j]) : -1;
-          float4 dA = make_float4(0.f, 0.f, 0.f, 0.f), cA = dA, dB = dA, cB = dA;
-          if (qA >= 0) { dA = __ldg(L.frame + 2 * qA); cA = __ldg(L.frame + 2 * qA + 1); }
-          if (qB >= 0) { dB = __ldg(L.frame + 2 * qB); cB = __ldg(L.frame + 2 * qB + 1); }
-          // the model points are read again from shared memory rather than
-          // held in registers across the gathers
-          asm volatile("" ::: "memory");
-          if (qA >= 0) {
-            examined += 1.f;
-            try_row(acc, s_c2w, s_pts[2 * i], s_pts[2 * i + 1], dA, cA, dist2, nthr);
-          }
-          if (qB >= 0) {
-            examined += 1.f;
-            try_row(acc, s_c2w, s_pts[2 * j], s_pts[2 * j + 1], dB, cB, dist2, nthr);
-          }
+        for (int q = 0; q < 4; ++q) {
+          const int i = (int)threadIdx.x + q * kFusedThreads;
+          pt[q].seen = i < n;
+          const float4 m = s_pts[2 * (pt[q].seen ? i : 0)];
+          const int px = associate_flat(s_w2c, L.cam, make_float3(m.x, m.y, m.z), pt[q].seen);
+          pt[q].f = load_point<WIDE>(L.frame + 2 * px);
         }
-        // the rest of the block's chunks, from global memory
-        for (int k = kc + warp; k < my_chunks; k += kWarps) {
-          const int p = ((int)blockIdx.x + k * G) * 32 + lane;
-          if (p >= npx) continue;
-          const float4 s = __ldg(L.model + 2 * p);
-          const float4 ns = __ldg(L.model + 2 * p + 1);
-          if (s.w == 0.f || ns.w == 0.f) continue;
-          const int q = associate(s_w2c, L.cam, s);
-          if (q < 0) continue;
-          examined += 1.f;
-          try_row(acc, s_c2w, s, ns, __ldg(L.frame + 2 * q), __ldg(L.frame + 2 * q + 1), dist2,
-                  nthr);
-        }
-        // pairwise sums: a recursive-halving exchange across the warp (lanes
-        // trade half of their remaining values each step, 31 shuffles for 32
-        // values) leaves lane v with the warp's sum of value v; then a tree
-        // over the block's warps. Value kVals is the examined-point count. A
-        // warp that examined no point (the coarse levels leave most warps
-        // idle) holds only +0 and writes its zeros directly.
-        if (!__any_sync(0xffffffffu, examined > 0.f)) {
-          s_red[warp][lane] = 0.f;
-        } else {
-          float r[32];
 #pragma unroll
-          for (int v = 0; v < 32; ++v) r[v] = v < kVals ? acc[v] : (v == kVals ? examined : 0.f);
+        for (int h = 0; h < 2; ++h) {
+          float acc[kVals];
+          float examined = 0.f;  // model points that project into the frame
 #pragma unroll
-          for (int sft = 16; sft >= 1; sft >>= 1) {
-            const bool upper = (lane & sft) != 0;
+          for (int v = 0; v < kVals; ++v) acc[v] = 0.f;
+          // the chain's first two cached points
 #pragma unroll
-            for (int i = 0; i < sft; ++i) {
-              float send = upper ? r[i] : r[i + sft];
-              float keep = upper ? r[i + sft] : r[i];
-              r[i] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
+          for (int r = 0; r < 2; ++r) {
+            BatchPoint &b = pt[2 * r + h];
+            // (the model point is read again from shared memory rather than
+            // held in registers across the gathers)
+            asm volatile("" ::: "memory");
+            const int i = (int)threadIdx.x + (2 * r + h) * kFusedThreads;
+            const float4 sp = s_pts[2 * (i < n ? i : 0)], np = s_pts[2 * (i < n ? i : 0) + 1];
+            b.s = make_float3(sp.x, sp.y, sp.z);
+            b.ns = make_float3(np.x, np.y, np.z);
+            float a[8];
+            batch_row(a, s_c2w, b, dist2, nthr);
+            batch_add(acc, a);
+            examined += b.seen ? 1.f : 0.f;
+          }
+          // its further ones
+          for (int i = (int)threadIdx.x + h * kFusedThreads + 2 * kFusedChains; i < n; i += kFusedChains) {
+            const int q = associate(s_w2c, L.cam, s_pts[2 * i]);
+            if (q < 0) continue;
+            examined += 1.f;
+            try_row(acc, s_c2w, s_pts[2 * i], s_pts[2 * i + 1], __ldg(L.frame + 2 * q),
+                    __ldg(L.frame + 2 * q + 1), dist2, nthr);
+          }
+          // the rest of the block's chunks, from global memory
+          for (int k = kc + warp + h * kWarps; k < my_chunks; k += kChainWarps) {
+            const int p = ((int)blockIdx.x + k * G) * 32 + lane;
+            if (p >= npx) continue;
+            const float4 s = __ldg(L.model + 2 * p);
+            const float4 ns = __ldg(L.model + 2 * p + 1);
+            if (s.w == 0.f || ns.w == 0.f) continue;
+            const int q = associate(s_w2c, L.cam, s);
+            if (q < 0) continue;
+            examined += 1.f;
+            try_row(acc, s_c2w, s, ns, __ldg(L.frame + 2 * q), __ldg(L.frame + 2 * q + 1), dist2,
+                    nthr);
+          }
+          // pairwise sums: a recursive-halving exchange across the warp (lanes
+          // trade half of their remaining values each step, 31 shuffles for 32
+          // values) leaves lane v with the warp's sum of value v; then a tree
+          // over the block's chain warps. Value kVals is the examined-point
+          // count. A warp that examined no point (the coarse levels leave most
+          // idle) holds only +0 and writes its zeros directly.
+          if (!__any_sync(0xffffffffu, examined > 0.f)) {
+            s_red[warp + h * kWarps][lane] = 0.f;
+          } else {
+            float r[32];
+#pragma unroll
+            for (int v = 0; v < 32; ++v) r[v] = v < kVals ? acc[v] : (v == kVals ? examined : 0.f);
+#pragma unroll
+            for (int sft = 16; sft >= 1; sft >>= 1) {
+              const bool upper = (lane & sft) != 0;
+#pragma unroll
+              for (int i = 0; i < sft; ++i) {
+                float send = upper ? r[i] : r[i + sft];
+                float keep = upper ? r[i + sft] : r[i];
+                r[i] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
+              }
             }
+            s_red[warp + h * kWarps][lane] = r[0];
           }
-          s_red[warp][lane] = r[0];
         }
         __syncthreads();
         const int buf = iter_global & 1;
         const unsigned seq = (epoch << kIterBits) | (unsigned)(iter_global + 1);
         if (warp == 0) {
-          float y[kWarps];
+          float y[kChainWarps];
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) y[w] = s_red[w][lane];
+          for (int w = 0; w < kChainWarps; ++w) y[w] = s_red[w][lane];
 #pragma unroll
-          for (int span = 1; span < kWarps; span *= 2)
+          for (int span = 1; span < kChainWarps; span *= 2)
 #pragma unroll
-            for (int w = 0; w + span < kWarps; w += 2 * span) y[w] += y[w + span];
+            for (int w = 0; w + span < kChainWarps; w += 2 * span) y[w] += y[w + span];
           // publish: each value with this iteration's sequence number in one
           // 64-bit store (no fence: a slot validates itself)
           if (lane <= kVals)
@@ -770,28 +909,36 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         // this iteration's grid barrier. Lane v of warp g reads value v of
         // rows g, g + 32, ...; a round re-reads only the slots not yet seen.
         {
-          constexpr int kPer = (kFusedMaxBlocks + kWarps - 1) / kWarps;
-          const int v = lane, grp = warp;
-          float vals[kPer];
-          unsigned pending = 0;
+          // (a warp reads two groups of up to ROWS rows)
+          const int v = lane;
+          float vals[2][ROWS];
+          unsigned pending[2] = {0u, 0u};
 #pragma unroll
-          for (int q = 0; q < kPer; ++q) {
-            vals[q] = 0.f;
-            if (v <= kVals && grp + q * kWarps < (int)gridDim.x) pending |= 1u << q;
-          }
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) {
+              vals[h][q] = 0.f;
+              if (v <= kVals && warp + h * kWarps + q * kChainWarps < (int)gridDim.x) pending[h] |= 1u << q;
+            }
           unsigned spins = 0;
           for (;;) {
+            // (every slot's load is issued before the first is looked at)
+            unsigned long long w[2][ROWS];
 #pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-              if (!((pending >> q) & 1u)) continue;
-              const unsigned long long w =
-                  ld_relaxed_gpu(&ws->fused_rows[buf][grp + q * kWarps][v]);
-              if ((unsigned)(w >> 32) == seq) {
-                vals[q] = __uint_as_float((unsigned)w);
-                pending &= ~(1u << q);
-              }
-            }
-            if (__all_sync(0xffffffffu, pending == 0u)) break;
+            for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                if ((pending[h] >> q) & 1u)
+                  w[h][q] = ld_relaxed_gpu(&ws->fused_rows[buf][warp + h * kWarps + q * kChainWarps][v]);
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                if (((pending[h] >> q) & 1u) && (unsigned)(w[h][q] >> 32) == seq) {
+                  vals[h][q] = __uint_as_float((unsigned)w[h][q]);
+                  pending[h] &= ~(1u << q);
+                }
+            if (__all_sync(0xffffffffu, (pending[0] | pending[1]) == 0u)) break;
             if (++spins > kSpinLimit ||
                 ((spins & 255u) == 0u && ld_acquire_gpu(reinterpret_cast<unsigned *>(&ws->error)))) {
               if (lane == 0) {
@@ -802,47 +949,45 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             }
             __nanosleep(32);
           }
-          float sum = 0.f, c = 0.f;
 #pragma unroll
-          for (int q = 0; q < kPer; ++q) {
-            float y = vals[q] - c;
-            float t = sum + y;
-            c = (t - sum) - y;
-            sum = t;
+          for (int h = 0; h < 2; ++h) {
+            float sum = 0.f, c = 0.f;
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) {
+              float y = vals[h][q] - c;
+              float t = sum + y;
+              c = (t - sum) - y;
+              sum = t;
+            }
+            s_red[warp + h * kWarps][v] = sum - c;
           }
-          s_red[grp][v] = sum - c;
         }
         // a wait that gave up (here or, later, in every other block) ends this
         // frame's tracking; the final status reads the workspace's flag
         __syncthreads();
         if (s_err) break;
         if (threadIdx.x < 32) {
-          float y[kWarps];
+          float y[kChainWarps];
 #pragma unroll
-          for (int w = 0; w < kWarps; ++w) y[w] = s_red[w][threadIdx.x];
+          for (int w = 0; w < kChainWarps; ++w) y[w] = s_red[w][threadIdx.x];
 #pragma unroll
-          for (int span = 1; span < kWarps; span *= 2)
+          for (int span = 1; span < kChainWarps; span *= 2)
 #pragma unroll
-            for (int w = 0; w + span < kWarps; w += 2 * span) y[w] += y[w + span];
+            for (int w = 0; w + span < kChainWarps; w += 2 * span) y[w] += y[w + span];
           s_tot[threadIdx.x] = y[0];
           __syncwarp();
-          double minpiv = 0.0;
-          float inc_rot = 0.f, inc_trans = 0.f;
           // (on success the warp also writes the new pose's rigid transforms)
-          const bool ok =
-              warp_solve_update(s_tot, s_pose, &minpiv, &inc_rot, &inc_trans, &s_c2w, &s_w2c);
+          SolveInfo info;
+          const bool solved = warp_solve_update(s_tot, s_sys, s_pose, &info, &s_c2w, &s_w2c);
           if (threadIdx.x == 0) {
-            s_its += 1;
-            s_inl = (int)s_tot[28];
-            s_examined = (int)s_tot[kVals];
-            s_res = (double)s_tot[27];
-            s_piv = minpiv;
-            if (!ok) {
+            s_info = info;
+            s_solved = solved;
+            if (!solved) {
               for (int i = 0; i < 16; ++i) s_pose[i] = ws->pose_init[i];
               s_stop = 1;
               pose_to_rigid(s_pose, &s_c2w, &s_w2c);
-            } else if (plan.stop_rot > 0.f && inc_rot < plan.stop_rot &&
-                       inc_trans < plan.stop_trans) {
+            } else if (plan.stop_rot > 0.f && info.inc_rot < plan.stop_rot &&
+                       info.inc_trans < plan.stop_trans) {
               s_conv = 1;  // converged at this level
             }
           }
@@ -856,7 +1001,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     if (pass == 1 || !warm || s_err) break;
     __syncthreads();  // every thread has left the level loop (it reads s_stop)
     if (threadIdx.x == 0) {
-      const bool keep = !s_stop && judge_keep(plan, ws->warm_pose, s_pose, s_res, s_inl, s_examined);
+      const bool keep = !s_stop && judge_keep(plan, ws->warm_pose, s_pose, (double)s_tot[27],
+                                           (int)s_tot[28], (int)s_tot[kVals]);
       s_warm = keep ? 1 : 2;
       if (!keep) {
         s_stop = 0;
@@ -876,14 +1022,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       for (int i = 0; i < 16; ++i) dst[i] = err ? ws->pose_init[i] : s_pose[i];
       *plan.hist_count = c + 1;
     }
-    ws->iterations = s_its;
+    ws->iterations = iter_global;
     if (stats) {
       stats->status = err ? 2 : (s_stop ? 1 : 0);
-      stats->inliers = s_inl;
-      stats->iterations = s_its;
+      stats->inliers = (int)s_tot[28];
+      stats->iterations = iter_global;
       stats->warm = warm ? s_warm : 0;
-      stats->residual_sq = s_res;
-      stats->min_pivot = s_piv;
+      stats->residual_sq = (double)s_tot[27];
+      stats->min_pivot = iter_global > 0 ? min_pivot(s_info, s_solved) : 0.0;
     }
   }
 }
@@ -986,6 +1132,14 @@ static bool icp_params_ok(const of_icp_params_t *p) {
   return p->dist_thresh_mm > 0.f;
 }
 
+// The fused kernel's instances: [0, 1] for grids of up to 160 blocks (5 rows a
+// group; a B200 has 148), [2, 3] for larger ones; the odd ones for frame
+// pyramids off a 32-byte boundary.
+constexpr int kFewRows = 5, kMostRows = (kFusedMaxBlocks + kChainWarps - 1) / kChainWarps;
+static const void *const kFusedKernels[4] = {
+    (const void *)k_icp_fused<true, kFewRows>, (const void *)k_icp_fused<false, kFewRows>,
+    (const void *)k_icp_fused<true, kMostRows>, (const void *)k_icp_fused<false, kMostRows>};
+
 // Launch shape of the fused kernel on the current device: every block
 // co-resident (cooperative launch), with room in shared memory for the
 // block's slice of the finest level's model points (up to kMaxCachePts).
@@ -1005,14 +1159,14 @@ static of_status_t fused_shape(const of_camera_t *cam, FusedShape *fs) {
   // The shared-memory opt-in belongs to the function in the current context:
   // it is set on every call (a host-side call), so that a context created
   // after cudaDeviceReset gets it too. The grid depends only on the device.
-  OF_CUDA_TRY(cudaFuncSetAttribute((const void *)k_icp_fused,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+  for (const void *k : kFusedKernels)
+    OF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
   {
     std::lock_guard<std::mutex> lock(mu);
     if (grid_of[dev] == 0) {
       int sms = 0, per_sm = 0;
       OF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      OF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_icp_fused,
+      OF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kFusedKernels[0],
                                                                 kFusedThreads, max_smem));
       grid_of[dev] = sms * (per_sm < 1 ? 1 : per_sm);
     }
@@ -1082,7 +1236,9 @@ static of_status_t icp_fused_launch(const of_camera_t *cam, const of_icp_params_
     if (st != OF_OK) return st;
   }
   void *args[] = {&plan, &pose, &ws, &stats};
-  OF_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_icp_fused, dim3(fs.grid),
+  const void *kern = kFusedKernels[(fs.grid > kFewRows * kChainWarps ? 2 : 0) +
+                                   (((uintptr_t)d_frame & 31u) != 0 ? 1 : 0)];
+  OF_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(fs.grid),
                                           dim3(kFusedThreads), args, fs.smem, s));
   return OF_OK;
 }
@@ -1159,14 +1315,13 @@ namespace {
 __global__ void __launch_bounds__(32) k_icp_solve_step(const float *__restrict__ sys, double *pose,
                                                        of_icp_stats_t *stats) {
   __shared__ float s_tot[32];
-  __shared__ double s_pose[16];
+  __shared__ double s_pose[16], s_sys[32];
   const int lane = threadIdx.x;
   s_tot[lane] = lane < kVals ? sys[lane] : 0.f;
   if (lane < 16) s_pose[lane] = pose[lane];
   __syncwarp();
-  double minpiv = 0.0;
-  float inc_rot = 0.f, inc_trans = 0.f;
-  const bool ok = warp_solve_update(s_tot, s_pose, &minpiv, &inc_rot, &inc_trans);
+  SolveInfo info;
+  const bool ok = warp_solve_update(s_tot, s_sys, s_pose, &info);
   if (ok && lane < 16) pose[lane] = s_pose[lane];
   if (lane == 0 && stats) {
     stats->status = ok ? 0 : 1;
@@ -1174,7 +1329,7 @@ __global__ void __launch_bounds__(32) k_icp_solve_step(const float *__restrict__
     stats->iterations = 1;
     stats->warm = 0;
     stats->residual_sq = (double)s_tot[27];
-    stats->min_pivot = minpiv;
+    stats->min_pivot = min_pivot(info, ok);
   }
 }
 }  // namespace
@@ -1280,89 +1435,6 @@ struct IcpJob {
   of_icp_stats_t *stats;
 };
 
-// A point of a pyramid (vertex, normal), one 32-byte load: the batch's
-// pyramids start at 256-byte boundaries.
-struct MapPoint {
-  float4 v, n;
-};
-__device__ __forceinline__ MapPoint ld_point(const float4 *p) {
-  MapPoint m;
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(m.v.x), "=f"(m.v.y), "=f"(m.v.z), "=f"(m.v.w), "=f"(m.n.x), "=f"(m.n.y), "=f"(m.n.z),
-        "=f"(m.n.w)
-      : "l"(p));
-  return m;
-}
-// 1 / z rounded to nearest for |z| in [2^-126, 2^126), without a branch: the
-// approximate reciprocal, a Newton step, and Markstein's final step (IBM
-// Journal of R&D 34, 1990), which rounds correctly from an approximation that
-// is right to within an ulp. Equal to __frcp_rn for every
-// mantissa, sign and exponent of that range (checked on B200 over all of them).
-__device__ __forceinline__ float recip_rn(float z) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(z));
-  y = __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
-  return __fmaf_rn(__fmaf_rn(-z, y, 1.f), y, y);
-}
-// associate() without a branch: the frame pixel (0 if none), and whether the
-// point projects into the frame.
-__device__ __forceinline__ int associate_flat(const Rigid &w2c, const Cam &cam, float3 s, bool &seen) {
-  const float3 sc = apply(w2c, s);
-  const float rz = recip_rn(sc.z);
-  const int pu = __float2int_rd(fmaf(cam.fx * sc.x, rz, cam.cx) + 0.5f);
-  const int pv = __float2int_rd(fmaf(cam.fy * sc.y, rz, cam.cy) + 0.5f);
-  seen = seen && !(sc.z >= -kEps) && (unsigned)pu < (unsigned)cam.w && (unsigned)pv < (unsigned)cam.h;
-  return seen ? pv * cam.w + pu : 0;
-}
-
-// A model point, the frame point at its pixel, and whether it has one.
-struct BatchPoint {
-  float3 s, ns;
-  MapPoint f;
-  bool seen;
-};
-__device__ __forceinline__ BatchPoint batch_frame(const MapPoint &m, bool live, const Rigid &w2c,
-                                                  const Cam &cam, const float4 *__restrict__ frame) {
-  BatchPoint b;
-  b.s = make_float3(m.v.x, m.v.y, m.v.z);
-  b.ns = make_float3(m.n.x, m.n.y, m.n.z);
-  b.seen = live && m.v.w != 0.f && m.n.w != 0.f;
-  const int q = associate_flat(w2c, cam, b.s, b.seen);
-  b.f = ld_point(frame + 2 * q);
-  return b;
-}
-// The point's row a[0..5], b = a[6] and inlier count a[7] (try_row's tests and
-// arithmetic); zeros when it is no inlier.
-__device__ __forceinline__ void batch_row(float (&a)[8], const Rigid &c2w, const BatchPoint &p,
-                                          float dist2, float nthr) {
-  const float3 s = p.s, ns = p.ns;
-  const float3 d = apply(c2w, make_float3(p.f.v.x, p.f.v.y, p.f.v.z));
-  const float3 nd = rotate(c2w, make_float3(p.f.n.x, p.f.n.y, p.f.n.z));
-  const float ex = d.x - s.x, ey = d.y - s.y, ez = d.z - s.z;
-  const float dn = nd.x * ns.x + nd.y * ns.y + nd.z * ns.z;
-  const bool ok = p.seen && p.f.v.w != 0.f && p.f.n.w != 0.f &&
-                  fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < dist2 && dn > nthr && dn < 1.f + kEps;
-  a[0] = ok ? ns.y * d.z - ns.z * d.y : 0.f;
-  a[1] = ok ? ns.z * d.x - ns.x * d.z : 0.f;
-  a[2] = ok ? ns.x * d.y - ns.y * d.x : 0.f;
-  a[3] = ok ? ns.x : 0.f;
-  a[4] = ok ? ns.y : 0.f;
-  a[5] = ok ? ns.z : 0.f;
-  a[6] = ok ? -(ns.x * ex + ns.y * ey + ns.z * ez) : 0.f;
-  a[7] = ok ? 1.f : 0.f;
-}
-__device__ __forceinline__ void batch_add(float *acc, const float (&a)[8]) {
-  int k = 0;
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int j = i; j < 6; ++j) { acc[k] = fmaf(a[i], a[j], acc[k]); ++k; }
-#pragma unroll
-  for (int i = 0; i < 6; ++i) acc[21 + i] = fmaf(a[i], a[6], acc[21 + i]);
-  acc[27] = fmaf(a[6], a[6], acc[27]);
-  acc[28] += a[7];
-}
-
 template <int CTAS>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTAS), 1)
     k_icp_batch(const IcpJob *__restrict__ jobs, const int *__restrict__ order, int njobs,
@@ -1374,8 +1446,10 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTA
   __shared__ float s_red[ROWS][32];
   __shared__ float s_part[2][CTAS][32];
   __shared__ float s_tot[32];
-  __shared__ int s_job, s_stop, s_conv, s_its, s_inl;
-  __shared__ double s_res, s_piv;
+  __shared__ double s_sys[32];
+  __shared__ SolveInfo s_info;  // of the stream's last solve (its sums stay in s_tot)
+  __shared__ bool s_solved;
+  __shared__ int s_job, s_stop, s_conv;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1396,9 +1470,8 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTA
       s_pose[threadIdx.x] = J.pose[threadIdx.x];
       s_init[threadIdx.x] = J.pose[threadIdx.x];
     }
-    if (threadIdx.x == 0) {
-      s_stop = 0; s_conv = 0; s_its = 0; s_inl = 0; s_res = 0.0; s_piv = 0.0;
-    }
+    if (threadIdx.x == 0) { s_stop = 0; s_conv = 0; }
+    if (threadIdx.x < 32) s_tot[threadIdx.x] = 0.f;
     __syncthreads();
     if (threadIdx.x == 0) pose_to_rigid(s_pose, &s_c2w, &s_w2c);
     __syncthreads();
@@ -1487,21 +1560,17 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTA
             for (int r = 0; r + span < CTAS; r += 2 * span) y[r] += y[r + span];
           s_tot[lane] = y[0];
           __syncwarp();
-          double minpiv = 0.0;
-          float inc_rot = 0.f, inc_trans = 0.f;
           // (on success the warp also writes the new pose's rigid transforms)
-          const bool ok =
-              warp_solve_update(s_tot, s_pose, &minpiv, &inc_rot, &inc_trans, &s_c2w, &s_w2c);
+          SolveInfo info;
+          const bool solved = warp_solve_update(s_tot, s_sys, s_pose, &info, &s_c2w, &s_w2c);
           if (lane == 0) {
-            s_its += 1;
-            s_inl = (int)s_tot[28];
-            s_res = (double)s_tot[27];
-            s_piv = minpiv;
-            if (!ok) {
+            s_info = info;
+            s_solved = solved;
+            if (!solved) {
               for (int i = 0; i < 16; ++i) s_pose[i] = s_init[i];
               s_stop = 1;
               pose_to_rigid(s_pose, &s_c2w, &s_w2c);
-            } else if (stop_rot > 0.f && inc_rot < stop_rot && inc_trans < stop_trans) {
+            } else if (stop_rot > 0.f && info.inc_rot < stop_rot && info.inc_trans < stop_trans) {
               s_conv = 1;
             }
           }
@@ -1515,11 +1584,11 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(batch_threads(CTA
       for (int i = 0; i < 16; ++i) J.pose[i] = s_pose[i];
       if (J.stats) {
         J.stats->status = s_stop ? 1 : 0;
-        J.stats->inliers = s_inl;
-        J.stats->iterations = s_its;
+        J.stats->inliers = (int)s_tot[28];
+        J.stats->iterations = iter;
         J.stats->warm = 0;
-        J.stats->residual_sq = s_res;
-        J.stats->min_pivot = s_piv;
+        J.stats->residual_sq = (double)s_tot[27];
+        J.stats->min_pivot = iter > 0 ? min_pivot(s_info, s_solved) : 0.0;
       }
     }
   }
