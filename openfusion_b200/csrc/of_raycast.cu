@@ -4,19 +4,28 @@
 // with the KinectFusion refinement it left commented out) is in of_raycast.cuh.
 #include "of_raycast.cuh"
 
+#include <numeric>
+
 bool of_camera_valid(const of_camera_t *c);
 bool of_volume_valid(const of_volume_desc_t *d);
 
 namespace {
 
+// The blocks take the image's tiles `stride` apart (coprime to their number,
+// near its golden section): the long rays, which lie together, neither start
+// last nor share an SM (fusion at 1024^3, 389 -> 380 us; 512^3 raycast 86.9 ->
+// 85.9). fp16's conversions leave room for 64 registers, which four blocks of
+// 256 on an SM need (380 -> 372 us).
 template <int STORAGE>
-__global__ void __launch_bounds__(256) k_raycast(const uint32_t *__restrict__ vol,
+__global__ void __launch_bounds__(256, STORAGE == OF_TSDF_F16 ? 4 : 1) k_raycast(const uint32_t *__restrict__ vol,
                                                  of_volume_desc_t desc, Cam cam,
                                                  of_raycast_params_t rp,
                                                  const double *__restrict__ pose,
                                                  float4 *__restrict__ pts, uint32_t *rgba,
-                                                 ModelLevels coarse) {
-  raycast_tile<STORAGE>(vol, desc, cam, rp, pose, pts, rgba, blockIdx.x, blockIdx.y, &coarse);
+                                                 ModelLevels coarse, unsigned stride) {
+  const unsigned lin = (unsigned)(((unsigned long long)(blockIdx.y * gridDim.x + blockIdx.x) * stride) %
+                                  (gridDim.x * gridDim.y));
+  raycast_tile<STORAGE>(vol, desc, cam, rp, pose, pts, rgba, lin % gridDim.x, lin / gridDim.x, &coarse);
 }
 
 // Model level l -> l+1 by subsampling pixel (2x, 2y): model points are used
@@ -217,11 +226,15 @@ extern "C" of_status_t of_raycast(const of_volume_desc_t *d, const void *vol,
     coarse.pts[l] = (float4 *)((char *)d_model + lay.points_offset[l]);
     coarse.w[l] = lay.width[l];
   }
+  const unsigned total = grid.x * grid.y;
+  unsigned stride = (unsigned)(0.6180339887 * total);
+  if (!stride) stride = 1;
+  while (std::gcd(stride, total) != 1) ++stride;
   if (d->storage == OF_TSDF_I16)
     k_raycast<OF_TSDF_I16><<<grid, blk, 0, s>>>((const uint32_t *)vol, *d, c, *rp, pose, pts, rgba,
-                                                coarse);
+                                                coarse, stride);
   else
     k_raycast<OF_TSDF_F16><<<grid, blk, 0, s>>>((const uint32_t *)vol, *d, c, *rp, pose, pts, rgba,
-                                                coarse);
+                                                coarse, stride);
   return of_launch_status();
 }

@@ -55,59 +55,74 @@ __device__ __forceinline__ int cell_index(float g, int n) {
   return (int)min(__float2uint_rd(g), (unsigned)(n - 2));
 }
 
-// Trilinear tsdf at a world position. Corner (i0, j0, k0) is clamped to
-// [0, n-2]; the seven other corners are the base address plus an axis step
-// that crosses into the next brick when the local coordinate is 7. Volume
-// indices fit in 32 bits (n <= 1024).
+// The cell of a world position: corner (ix, iy, iz), clamped to [0, n-2], its
+// word in the volume and the position's fractions. The seven other corners are
+// that word plus an axis step that crosses into the next brick when the local
+// coordinate is 7. Volume indices fit in 32 bits (n <= 1024).
+template <int STORAGE>
+struct Cell {
+  int ix, iy, iz;
+  float fx, fy, fz;
+  unsigned base;
+  __device__ __forceinline__ Cell(int n, int nb, float org, float inv_vs, float px, float py, float pz) {
+    // fp16 volumes: x and y positions in one instruction (the raycast at 1024^3
+    // 178 -> 154 us; int16's is 3 % slower that way and keeps the scalar form)
+    float gx, gy;
+    if (STORAGE == OF_TSDF_F16) {
+      const float2 g = fma2(sub2(make_float2(px, py), dup2(org)), dup2(inv_vs), dup2(-0.5f));
+      gx = g.x;
+      gy = g.y;
+    } else {
+      gx = fmaf(px - org, inv_vs, -0.5f);
+      gy = fmaf(py - org, inv_vs, -0.5f);
+    }
+    const float gz = fmaf(pz - org, inv_vs, -0.5f);
+    ix = cell_index(gx, n); iy = cell_index(gy, n); iz = cell_index(gz, n);
+    if (STORAGE == OF_TSDF_F16) {
+      const float2 f = sub2(make_float2(gx, gy), make_float2((float)ix, (float)iy));
+      fx = f.x;
+      fy = f.y;
+    } else {
+      fx = gx - (float)ix;
+      fy = gy - (float)iy;
+    }
+    fz = gz - (float)iz;
+    base = ((((unsigned)(ix >> 3) * nb + (unsigned)(iy >> 3)) * nb + (unsigned)(iz >> 3)) << 9) |
+           (unsigned)(((ix & 7) << 6) | ((iy & 7) << 3) | (iz & 7));
+  }
+  __device__ __forceinline__ void load(const uint32_t *__restrict__ vol, int nb, uint32_t (&w)[8]) const {
+    const unsigned dx = (ix & 7) == 7 ? (unsigned)nb * nb * 512u - 448u : 64u;
+    const unsigned dy = (iy & 7) == 7 ? (unsigned)nb * 512u - 56u : 8u;
+    const unsigned dz = (iz & 7) == 7 ? 505u : 1u;
+    const uint32_t *p0 = vol + base;
+    w[0] = __ldg(p0);
+    w[1] = __ldg(p0 + dz);
+    w[2] = __ldg(p0 + dy);
+    w[3] = __ldg(p0 + dy + dz);
+    w[4] = __ldg(p0 + dx);
+    w[5] = __ldg(p0 + dx + dz);
+    w[6] = __ldg(p0 + dx + dy);
+    w[7] = __ldg(p0 + dx + dy + dz);
+  }
+  __device__ __forceinline__ float value(const uint32_t (&w)[8]) const {
+    float c[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = ray_value<STORAGE>(w[i]);
+    const float c00 = fmaf(fz, c[1] - c[0], c[0]), c01 = fmaf(fz, c[3] - c[2], c[2]);
+    const float c10 = fmaf(fz, c[5] - c[4], c[4]), c11 = fmaf(fz, c[7] - c[6], c[6]);
+    const float c0 = fmaf(fy, c01 - c00, c00), c1 = fmaf(fy, c11 - c10, c10);
+    return fmaf(fx, c1 - c0, c0) * ray_scale<STORAGE>();
+  }
+};
+
+// Trilinear tsdf at a world position.
 template <int STORAGE>
 __device__ __forceinline__ float trilinear(const uint32_t *__restrict__ vol, int n, int nb,
-                                           float org, float inv_vs, float px, float py, float pz,
-                                           int3 *cell = nullptr) {
-  // fp16 volumes: x and y positions in one instruction (the raycast at 1024^3
-  // 178 -> 154 us; int16's is 3 % slower that way and keeps the scalar form)
-  float gx, gy;
-  if (STORAGE == OF_TSDF_F16) {
-    const float2 g = fma2(sub2(make_float2(px, py), dup2(org)), dup2(inv_vs), dup2(-0.5f));
-    gx = g.x;
-    gy = g.y;
-  } else {
-    gx = fmaf(px - org, inv_vs, -0.5f);
-    gy = fmaf(py - org, inv_vs, -0.5f);
-  }
-  float gz = fmaf(pz - org, inv_vs, -0.5f);
-  int ix = cell_index(gx, n), iy = cell_index(gy, n), iz = cell_index(gz, n);
-  float fx, fy;
-  if (STORAGE == OF_TSDF_F16) {
-    const float2 f = sub2(make_float2(gx, gy), make_float2((float)ix, (float)iy));
-    fx = f.x;
-    fy = f.y;
-  } else {
-    fx = gx - (float)ix;
-    fy = gy - (float)iy;
-  }
-  float fz = gz - (float)iz;
-  if (cell) *cell = make_int3(ix, iy, iz);
-  unsigned base = ((((unsigned)(ix >> 3) * nb + (unsigned)(iy >> 3)) * nb + (unsigned)(iz >> 3)) << 9) |
-                  (unsigned)(((ix & 7) << 6) | ((iy & 7) << 3) | (iz & 7));
-  unsigned dx = (ix & 7) == 7 ? (unsigned)nb * nb * 512u - 448u : 64u;
-  unsigned dy = (iy & 7) == 7 ? (unsigned)nb * 512u - 56u : 8u;
-  unsigned dz = (iz & 7) == 7 ? 505u : 1u;
-  const uint32_t *p0 = vol + base;
-  float c000 = ray_value<STORAGE>(__ldg(p0));
-  float c001 = ray_value<STORAGE>(__ldg(p0 + dz));
-  float c010 = ray_value<STORAGE>(__ldg(p0 + dy));
-  float c011 = ray_value<STORAGE>(__ldg(p0 + dy + dz));
-  float c100 = ray_value<STORAGE>(__ldg(p0 + dx));
-  float c101 = ray_value<STORAGE>(__ldg(p0 + dx + dz));
-  float c110 = ray_value<STORAGE>(__ldg(p0 + dx + dy));
-  float c111 = ray_value<STORAGE>(__ldg(p0 + dx + dy + dz));
-  float c00 = fmaf(fz, c001 - c000, c000);
-  float c01 = fmaf(fz, c011 - c010, c010);
-  float c10 = fmaf(fz, c101 - c100, c100);
-  float c11 = fmaf(fz, c111 - c110, c110);
-  float c0 = fmaf(fy, c01 - c00, c00);
-  float c1 = fmaf(fy, c11 - c10, c10);
-  return fmaf(fx, c1 - c0, c0) * ray_scale<STORAGE>();
+                                           float org, float inv_vs, float px, float py, float pz) {
+  const Cell<STORAGE> c(n, nb, org, inv_vs, px, py, pz);
+  uint32_t w[8];
+  c.load(vol, nb, w);
+  return c.value(w);
 }
 
 // Central differences of the trilinear field one voxel apart along each axis
@@ -198,15 +213,26 @@ __device__ __noinline__ void write_coarse(const ModelLevels &coarse, int x, int 
   }
 }
 
-// The per-launch constants of a raycast at `pose` (one thread computes them).
+// The per-launch constants of a raycast at `pose`, one a thread: the pose's
+// twelve entries (as pose_to_rigid gives them), then the box and the voxel's
+// reciprocal, so that the block waits once for the loads and the divisions.
 __device__ __forceinline__ void ray_setup(const double *__restrict__ pose,
-                                          const of_volume_desc_t &desc, RaySetup *S) {
-  pose_to_rigid(pose, &S->c2w, nullptr);
-  S->cpos[0] = S->c2w.t[0]; S->cpos[1] = S->c2w.t[1]; S->cpos[2] = S->c2w.t[2];
-  double vs = (double)desc.size_mm / desc.resolution;
-  S->lo = (float)(-0.5 * desc.size_mm + 0.5 * vs + 1e-3);
-  S->hi = (float)(0.5 * desc.size_mm - 0.5 * vs - 1e-3);
-  S->inv_vs = (float)(1.0 / vs);
+                                          const of_volume_desc_t &desc, RaySetup *S, int i) {
+  if (i < 12) {
+    const float v = (float)pose[i];
+    const int r = i >> 2, c = i & 3;
+    if (c < 3) {
+      S->c2w.r[3 * r + c] = v;
+    } else {
+      S->c2w.t[r] = v;
+      S->cpos[r] = v;
+    }
+  } else if (i < 15) {
+    const double vs = (double)desc.size_mm / desc.resolution;
+    if (i == 12) S->lo = (float)(-0.5 * desc.size_mm + 0.5 * vs + 1e-3);
+    if (i == 13) S->hi = (float)(0.5 * desc.size_mm - 0.5 * vs - 1e-3);
+    if (i == 14) S->inv_vs = (float)(1.0 / vs);
+  }
 }
 
 // The ray of pixel (x, y), inside the image: march, refine, normal; writes
@@ -262,105 +288,89 @@ __device__ __forceinline__ void raycast_pixel(const uint32_t *__restrict__ vol,
     // the axis planes: that axis bounds no jump)
     const bool ux = fabsf(dir.x) > 1e-12f, uy = fabsf(dir.y) > 1e-12f, uz = fabsf(dir.z) > 1e-12f;
     const float rdx = ux ? 1.0f / dir.x : 0.f, rdy = uy ? 1.0f / dir.y : 0.f, rdz = uz ? 1.0f / dir.z : 0.f;
-    float t = t0;
-    float fp = 1.0f;
-    bool sampled = false;
-    int cur_b = -1, cur_s = -1;  // brick / super-brick the march is in, and their flags
-    bool cur_flag = false, cur_sflag = false;
-    // the clamped cell base of the position at t when the last sample was
-    // taken there (the same expression as below, so the same brick)
-    int3 cell = make_int3(0, 0, 0);
-    bool have_cell = false;
-    for (int it = 0; it < (1 << 16); ++it) {
-      if (!have_cell) {
-        const float px = fmaf(t, dir.x, ox), py = fmaf(t, dir.y, oy), pz = fmaf(t, dir.z, oz);
-        cell.x = cell_index(fmaf(px - org, inv_vs, -0.5f), n);
-        cell.y = cell_index(fmaf(py - org, inv_vs, -0.5f), n);
-        cell.z = cell_index(fmaf(pz - org, inv_vs, -0.5f), n);
-      }
-      have_cell = false;
-      const int bi = cell.x >> 3, bj = cell.y >> 3, bk = cell.z >> 3;
-      // (cell indices are clamped to >= 0: unsigned division is a shift)
+    // One point of the ray a pass: its brick's and super-brick's flags and (where
+    // a sample is due) the cell's eight corners are requested together, so a
+    // pass waits for memory once, whatever mix of empty and sampled points the
+    // warp's lanes are at. The kernel is bound by the passes' latency as much as
+    // by issue: a warp's longest ray takes 20 passes in the median, 97 at most,
+    // and the last warps run on nearly empty SMs. 640x480 rays into 512^3: 97.6
+    // us with the flags looked up before the sample, 85.5 together. (Slower: the
+    // next free-space sample read ahead, 98 .. 108; every lane's skips finished
+    // before the samples, 124; indices from FP32 additions, 83.5 here but the
+    // 16-stream step 1.5 % slower.)
+    float t = t0, fp = 1.0f;  // the last point and its sample
+    float tn = t0, ta = 0.f, tb = 0.f, fa = 0.f, fb = 0.f;
+    bool due = true;       // tn's sample is not known to be +1
+    bool stepped = false;  // tn was reached by a step from t
+    for (int it = 0; it <= (1 << 16); ++it) {
+      const Cell<STORAGE> c(n, nb, org, inv_vs, fmaf(tn, dir.x, ox), fmaf(tn, dir.y, oy),
+                            fmaf(tn, dir.z, oz));
+      const int bi = c.ix >> 3, bj = c.iy >> 3, bk = c.iz >> 3;
+      // (cell indices are >= 0: unsigned division is a shift)
       const int si = (int)((unsigned)bi / kSuper), sj = (int)((unsigned)bj / kSuper),
                 sk = (int)((unsigned)bk / kSuper);
-      const int sidx = (si * ns + sj) * ns + sk;
-      if (sidx != cur_s) {
-        cur_s = sidx;
-        cur_sflag = __ldg(sflags + sidx) != 0;
-      }
-      bool skip = !cur_sflag;
-      if (!skip) {
-        const int b = (bi * nb + bj) * nb + bk;
-        if (b != cur_b) {
-          cur_b = b;
-          cur_flag = __ldg(flags + b) != 0;
+      const uint8_t sf = __ldg(sflags + (si * ns + sj) * ns + sk), bf = __ldg(flags + (c.base >> 9));
+      uint32_t w[8] = {};
+      if (due) c.load(vol, nb, w);
+      const float f = due ? c.value(w) : 1.0f;
+      if (stepped) {
+        if (fp > 0.f && f <= 0.f) {
+          ta = t; fa = fp; tb = tn; fb = f;
+          hit = true;
+          break;
         }
-        skip = !cur_flag;
+        if (fp < 0.f && f > 0.f) break;  // back face
       }
-      if (skip) {
+      t = tn;
+      fp = f;
+      if (!(sf && bf)) {
         // every sample with its cell base in this brick (or, when the
         // super-brick's flag is clear, in this super-brick) reads exactly +1:
         // jump just past the region; the landing cell is +1 as well. The
         // region of cell bases [8b, 8b + 8) along an axis is
         // p in [org + vs (8b + 0.5), org + vs (8b + 8.5)); R = 32 for a
         // super-brick.
-        const float R = cur_sflag ? 8.0f : (float)(8 * kSuper);
-        const int ci = cur_sflag ? bi : si, cj = cur_sflag ? bj : sj, ck = cur_sflag ? bk : sk;
+        const float R = sf ? 8.0f : (float)(8 * kSuper);
+        const int ci = sf ? bi : si, cj = sf ? bj : sj, ck = sf ? bk : sk;
         const float rvs = R * vs, h = org + 0.5f * vs;
         float te = 1e30f;
         if (ux) te = fminf(te, (fmaf(rvs, (float)(dir.x > 0.f ? ci + 1 : ci), h) - ox) * rdx);
         if (uy) te = fminf(te, (fmaf(rvs, (float)(dir.y > 0.f ? cj + 1 : cj), h) - oy) * rdy);
         if (uz) te = fminf(te, (fmaf(rvs, (float)(dir.z > 0.f ? ck + 1 : ck), h) - oz) * rdz);
-        t = fmaxf(te, t) + eps;
-        fp = 1.0f;
-        sampled = true;
-        if (t > t1) break;
-        continue;
+        tn = fmaxf(te, t) + eps;
+        due = stepped = false;
+      } else {
+        tn = t + (fp > 0.f ? fmaxf(min_step, far_k * fp) : min_step);
+        due = stepped = true;
       }
-      if (!sampled) {
-        fp = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(t, dir.x, ox), fmaf(t, dir.y, oy),
-                                fmaf(t, dir.z, oz));
-        sampled = true;
-      }
-      float step = fp > 0.f ? fmaxf(min_step, far_k * fp) : min_step;
-      float tn = t + step;
       if (tn > t1) break;
-      float fn = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(tn, dir.x, ox),
-                                    fmaf(tn, dir.y, oy), fmaf(tn, dir.z, oz), &cell);
-      if (fp > 0.f && fn <= 0.f) {
-        float ta = t, fa = fp, tb = tn, fb = fn;
-        // shrink a long bracket with minimum steps from its positive end, so
-        // the refined root does not depend on where the march samples fell
-        while (tb - ta > min_step * 1.0001f) {
-          float tm = ta + min_step;
-          float fm = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(tm, dir.x, ox),
-                                        fmaf(tm, dir.y, oy), fmaf(tm, dir.z, oz));
-          if (fm > 0.f) { ta = tm; fa = fm; } else { tb = tm; fb = fm; break; }
-        }
-        // Illinois regula falsi on the trilinear field
-        int side = 0;
-        for (int r = 0; r < rp.refine_iters; ++r) {
-          float tm = fmaf(tb - ta, fa / (fa - fb), ta);
-          float fm = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(tm, dir.x, ox),
-                                        fmaf(tm, dir.y, oy), fmaf(tm, dir.z, oz));
-          if (fm > 0.f) {
-            ta = tm; fa = fm;
-            if (side == 1) fb *= 0.5f;
-            side = 1;
-          } else {
-            tb = tm; fb = fm;
-            if (side == -1) fa *= 0.5f;
-            side = -1;
-          }
-        }
-        ts = fmaf(tb - ta, fa / (fa - fb), ta);
-        hit = true;
-        break;
+    }
+    if (hit) {
+      // shrink a long bracket with minimum steps from its positive end, so
+      // the refined root does not depend on where the march samples fell
+      while (tb - ta > min_step * 1.0001f) {
+        float tm = ta + min_step;
+        float fm = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(tm, dir.x, ox),
+                                      fmaf(tm, dir.y, oy), fmaf(tm, dir.z, oz));
+        if (fm > 0.f) { ta = tm; fa = fm; } else { tb = tm; fb = fm; break; }
       }
-      if (fp < 0.f && fn > 0.f) break;  // back face
-      t = tn;
-      fp = fn;
-      have_cell = true;
+      // Illinois regula falsi on the trilinear field
+      int side = 0;
+      for (int r = 0; r < rp.refine_iters; ++r) {
+        float tm = fmaf(tb - ta, fa / (fa - fb), ta);
+        float fm = trilinear<STORAGE>(vol, n, nb, org, inv_vs, fmaf(tm, dir.x, ox),
+                                      fmaf(tm, dir.y, oy), fmaf(tm, dir.z, oz));
+        if (fm > 0.f) {
+          ta = tm; fa = fm;
+          if (side == 1) fb *= 0.5f;
+          side = 1;
+        } else {
+          tb = tm; fb = fm;
+          if (side == -1) fa *= 0.5f;
+          side = -1;
+        }
+      }
+      ts = fmaf(tb - ta, fa / (fa - fb), ta);
     }
   }
   const size_t p = (size_t)y * cam.w + x;
@@ -401,7 +411,7 @@ __device__ __forceinline__ void raycast_tile(const uint32_t *__restrict__ vol,
                                              float4 *__restrict__ pts, uint32_t *rgba, int bx,
                                              int by, const ModelLevels *coarse = nullptr) {
   __shared__ RaySetup S;
-  if (threadIdx.x == 0 && threadIdx.y == 0) ray_setup(pose, desc, &S);
+  ray_setup(pose, desc, &S, (int)(threadIdx.y * blockDim.x + threadIdx.x));
   __syncthreads();
   const int x = bx * blockDim.x + threadIdx.x;
   const int y = by * blockDim.y + threadIdx.y;
