@@ -70,10 +70,19 @@ constexpr long fw_off(int l) {
 }
 constexpr int kFwFrags = fw_first(6);
 // Input-gradient fragments of conv2..4: one uint2 a lane for each (m tile, k8
-// step), m = ci, k = (co, tap): {(g, t) | (g + 8, t) << 16, (g, t + 4) |
-// (g + 8, t + 4) << 16}.
+// step), m = ci: {(g, t) | (g + 8, t) << 16, (g, t + 4) | (g + 8, t + 4) << 16}.
+// An input pixel of parity class (py, px) = (class / 2, class % 2) is reached
+// by 1, 2, 2 or 4 of the nine taps: the steps hold the four classes in turn,
+// each with its own taps alone, k = (co, tap of the class).
 constexpr int bw_mt(int l) { return kConv[l].ci / 16; }
 constexpr int bw_ks(int l) { return kConv[l].co * 9 / 8; }
+__host__ __device__ constexpr int bw_taps(int cls) { return (1 + (cls >> 1)) * (1 + (cls & 1)); }
+// The class's first step, in units of co / 8, and the class such a unit is of.
+__host__ __device__ constexpr int bw_before(int cls) { return cls == 0 ? 0 : 2 * cls - 1; }
+__host__ __device__ constexpr int bw_class(int unit) { return (unit + 1) / 2 < 3 ? (unit + 1) / 2 : 3; }
+// Tap j of a class, along y and x: 1 where the parity is even, else 0 and 2.
+__host__ __device__ constexpr int bw_tap_y(int cls, int j) { return cls >> 1 ? j / (1 + (cls & 1)) * 2 : 1; }
+__host__ __device__ constexpr int bw_tap_x(int cls, int j) { return cls & 1 ? j % 2 * 2 : 1; }
 constexpr int bw_first(int l) { return l <= 1 ? 0 : bw_first(l - 1) + bw_mt(l - 1) * bw_ks(l - 1); }
 constexpr int kBwFrags = bw_first(4);
 static_assert(fw_ks(1) * 16 == fw_k(1) && fw_ks(2) * 16 == fw_k(2) && fw_ks(3) * 16 == fw_k(3) &&
@@ -96,8 +105,12 @@ template <int L>
 __device__ __forceinline__ uint2 bw_frag(const bf16 *pw, int f, int lane) {
   const unsigned short *w = reinterpret_cast<const unsigned short *>(pw + fw_off(L));
   const int mt = f / bw_ks(L), ks = f % bw_ks(L), g = lane >> 2, t = lane & 3;
-  auto el = [&](int m, int k) -> uint32_t { return w[((k / 9) * kConv[L].ci + m) * 9 + k % 9]; };
-  const int m = mt * 16 + g, k = ks * 8 + t;
+  const int cls = bw_class(ks / (kConv[L].co / 8));
+  auto el = [&](int m, int k) -> uint32_t {
+    const int j = k % bw_taps(cls);
+    return w[((k / bw_taps(cls)) * kConv[L].ci + m) * 9 + bw_tap_y(cls, j) * 3 + bw_tap_x(cls, j)];
+  };
+  const int m = mt * 16 + g, k = (ks - kConv[L].co / 8 * bw_before(cls)) * 8 + t;
   return make_uint2(el(m, k) | el(m + 8, k) << 16, el(m, k + 4) | el(m + 8, k + 4) << 16);
 }
 
@@ -540,25 +553,30 @@ constexpr int kFcBiasBlocks = (kF1Out + kF2Out + 31) / 32;
 // Layer L's input gradient from the gradient at its (masked) output, stride 2:
 // input pixel (iy, ix) = (2r + py, 2c + px) takes tap (ky, kx) from output
 // pixel (r + dy, c + dx) with, per axis, parity 0: tap 1, offset 0; parity 1:
-// tap 0, offset 1 and tap 2, offset 0; the other taps contribute zeros. The n
-// tiles hold pixels of one parity class, so a tap's offset is the same for all
-// of them; a tap that does not reach the class points into a plane of zeros
-// (its products stay in the sum, in their place). Gradient planes:
-// [co][image][ho + 1][wo + 1], the last row and column zero, and one zero
-// plane after the last channel.
+// tap 0, offset 1 and tap 2, offset 0. The n tiles hold pixels of one parity
+// class, so that all of a tile take the same taps, 9 of the 36 (class, tap)
+// pairs in all. Gradient planes: [co][image][ho + 1][wo + 1], the last row and
+// column zero; a channel's stride is padded to the size with the fewest bank
+// conflicts between a tile's 8 pixels and 4 taps (a gather of two images 1.56 ..
+// 1.78 wavefronts unpadded, 1.16 .. 1.33 so).
 constexpr int gplane_w(int l) { return kConv[l].wo + 1; }
 constexpr int gplane_n(int l) { return (kConv[l].ho + 1) * (kConv[l].wo + 1); }
+constexpr int gplane_s(int l, int ni) {
+  return ni * gplane_n(l) + (ni == 2 ? (l == 1 ? 12 : l == 2 ? 10 : 20) : (l == 1 ? 0 : l == 2 ? 8 : 18));
+}
 template <int L, int NI>
 __device__ __forceinline__ void fill_bwd_taps(ushort2 *tab) {
-  static_assert((kConv[L].co + 1) * NI * gplane_n(L) < 65536, "16-bit offsets");
-  auto offset = [](int cls, int k) {
-    const int co = k / 9, ky = (k % 9) / 3, kx = k % 3, py = cls >> 1, px = cls & 1;
-    if ((py ? ky == 1 : ky != 1) || (px ? kx == 1 : kx != 1)) return kConv[L].co * NI * gplane_n(L);
-    return co * NI * gplane_n(L) + (py && ky == 0 ? gplane_w(L) : 0) + (px && kx == 0 ? 1 : 0);
-  };
-  for (int i = threadIdx.x; i < 4 * bw_ks(L) * 4; i += kTrThreads) {
-    const int t = i & 3, s = (i >> 2) % bw_ks(L), cls = (i >> 2) / bw_ks(L);
-    tab[i] = make_ushort2(offset(cls, s * 8 + t), offset(cls, s * 8 + t + 4));
+  static_assert(kConv[L].co * gplane_s(L, NI) < 65536, "16-bit offsets");
+  for (int i = threadIdx.x; i < bw_ks(L) * 4; i += kTrThreads) {
+    const int cls = bw_class((i >> 2) / (kConv[L].co / 8));
+    auto offset = [&](int k) {
+      const int j = k % bw_taps(cls);
+      return k / bw_taps(cls) * gplane_s(L, NI) +
+             (cls >> 1 && bw_tap_y(cls, j) == 0 ? gplane_w(L) : 0) +
+             (cls & 1 && bw_tap_x(cls, j) == 0 ? 1 : 0);
+    };
+    const int k = ((i >> 2) - kConv[L].co / 8 * bw_before(cls)) * 8 + (i & 3);
+    tab[i] = make_ushort2(offset(k), offset(k + 4));
   }
 }
 
@@ -573,36 +591,41 @@ __device__ __forceinline__ void conv_bwd_layer(const float *__restrict__ s_g,
   constexpr int KS = bw_ks(L), PL = gplane_n(L), PW = gplane_w(L), MU = bw_mt(L) / MT;
   constexpr int MAXPX = NI * ((c.hi + 1) / 2) * ((c.wi + 1) / 2);
   constexpr int NU = ((MAXPX + 7) / 8 + NT - 1) / NT;
-  static_assert(c.wi % 2 == 0 && bw_mt(L) % MT == 0 && KS % 4 == 0, "unit shape");
+  static_assert(NI <= 2 && c.wi % 2 == 0 && bw_mt(L) % MT == 0 && c.co % 32 == 0, "unit shape");
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int u = threadIdx.x >> 5; u < 4 * NU * MU; u += kTrWarps) {
-    const int mu = u % MU, cls = (u / MU) & 3, nu = u / (4 * MU);
+  // longest units first, dealt to the warps there and back
+  const int wp = threadIdx.x >> 5;
+  for (int r = 0; r * kTrWarps < 4 * NU * MU; ++r) {
+    const int u = r * kTrWarps + (r & 1 ? kTrWarps - 1 - wp : wp);
+    if (u >= 4 * NU * MU) continue;
+    const int cls = 3 - u / (NU * MU), mu = u % MU, nu = u / MU % NU;
+    const int first = c.co / 8 * bw_before(cls), steps = c.co / 8 * bw_taps(cls);
     const int py = cls >> 1, px = cls & 1;
     const int nc = c.wi / 2, cnt = ((c.hi + 1 - py) / 2) * nc;
     if (nu * NT * 8 >= NI * cnt) continue;
     int nb[NT];
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const int n = min((nu * NT + j) * 8 + g, NI * cnt - 1), img = n / cnt, p = n % cnt;
+      const int n = min((nu * NT + j) * 8 + g, NI * cnt - 1), img = NI == 2 && n >= cnt, p = n - img * cnt;
       nb[j] = img * PL + (p / nc) * PW + p % nc;
     }
     float acc[MT][NT][4] = {};
-    const uint2 *fa = bw + ((size_t)(bw_first(L) + mu * MT * KS)) * 32 + lane;
-    const ushort2 *ct = tab + cls * KS * 4 + t;
+    const uint2 *fa = bw + ((size_t)(bw_first(L) + mu * MT * KS + first)) * 32 + lane;
+    const ushort2 *ct = tab + first * 4 + t;
     // four steps of weights ahead
     uint2 nxt[4][MT];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int m = 0; m < MT; ++m) nxt[i][m] = __ldg(fa + (m * KS + i) * 32);
-    for (int s = 0; s < KS; s += 4)
+    for (int s = 0; s < steps; s += 4)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         uint2 a[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
           a[m] = nxt[i][m];
-          if (s + i + 4 < KS) nxt[i][m] = __ldg(fa + (m * KS + s + i + 4) * 32);
+          if (s + i + 4 < steps) nxt[i][m] = __ldg(fa + (m * KS + s + i + 4) * 32);
         }
         const ushort2 o = ct[(s + i) * 4];
 #pragma unroll
@@ -618,7 +641,7 @@ __device__ __forceinline__ void conv_bwd_layer(const float *__restrict__ s_g,
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int n = (nu * NT + j) * 8 + 2 * t + h, img = n / cnt, p = n % cnt;
+        const int n = (nu * NT + j) * 8 + 2 * t + h, img = NI == 2 && n >= cnt, p = n - img * cnt;
         if (n >= NI * cnt || img >= nimg) continue;
         const int y = 2 * (p / nc) + py, x = 2 * (p % nc) + px;
 #pragma unroll
@@ -629,7 +652,7 @@ __device__ __forceinline__ void conv_bwd_layer(const float *__restrict__ s_g,
             const size_t o = ((size_t)img * c.ci + ci) * (c.hi * c.wi) + y * c.wi + x;
             const float v = bf(act[o]) > 0.f ? to_tf32(acc[m][j][2 * r + h]) : 0.f;
             gin[o] = v;
-            if constexpr (L > 1) s_out[(ci * NI + img) * gplane_n(L - 1) + y * gplane_w(L - 1) + x] = v;
+            if constexpr (L > 1) s_out[ci * gplane_s(L - 1, NI) + img * gplane_n(L - 1) + y * gplane_w(L - 1) + x] = v;
           }
       }
   }
@@ -637,17 +660,21 @@ __device__ __forceinline__ void conv_bwd_layer(const float *__restrict__ s_g,
 
 template <int NI>
 struct BwdSmem {
-  alignas(16) float g4[129 * NI * gplane_n(3)];
-  alignas(16) float g3[65 * NI * gplane_n(2)];
-  alignas(16) float g2[33 * NI * gplane_n(1)];
-  alignas(16) ushort2 t3[4 * bw_ks(3) * 4], t2[4 * bw_ks(2) * 4], t1[4 * bw_ks(1) * 4];
+  alignas(16) float g4[128 * gplane_s(3, NI)];
+  alignas(16) float g3[64 * gplane_s(2, NI)];
+  alignas(16) float g2[32 * gplane_s(1, NI)];
+  alignas(16) ushort2 t3[bw_ks(3) * 4], t2[bw_ks(2) * 4], t1[bw_ks(1) * 4];
 };
 static_assert(sizeof(BwdSmem<2>) <= 227 * 1024 && sizeof(BwdSmem<1>) <= 113 * 1024, "shared memory");
 
 // The input gradients of conv4, conv3 and conv2 of NI images at a time, one
 // block; each is masked by the ReLU below it and rounded to TF32, which is
-// how the next layer and the weight gradients read it. Bound by the tensor
-// pipe's TF32 rate and the shared-memory gathers that feed it.
+// how the next layer and the weight gradients read it. Bound by latency and
+// issue with 16 warps an SM (tensor pipe 16 %, issue slots 40 %): about 20
+// instructions a tile product for gathers, weight unpacking and the scattered
+// stores. 256 pairs: 113 us with all nine taps of every class, 60 with each
+// class's own (two single-image blocks an SM, or 20 or 24 warps, spill: no
+// faster).
 template <int NI>
 __global__ void __launch_bounds__(kTrThreads) k_conv_dgrad(const float *__restrict__ g4,
                                                            const uint2 *__restrict__ bw, int batch,
@@ -671,17 +698,17 @@ __global__ void __launch_bounds__(kTrThreads) k_conv_dgrad(const float *__restri
     constexpr int HW = kConv[3].ho * kConv[3].wo;
     for (int i = threadIdx.x; i < NI * (int)kAct3; i += kTrThreads) {
       const int img = i / (int)kAct3, co = (i / HW) % 128, p = i % HW;
-      S.g4[(co * NI + img) * gplane_n(3) + (p / kConv[3].wo) * gplane_w(3) + p % kConv[3].wo] =
+      S.g4[co * gplane_s(3, NI) + img * gplane_n(3) + (p / kConv[3].wo) * gplane_w(3) + p % kConv[3].wo] =
           img < n ? __ldg(g4 + b * kAct3 + i) : 0.f;
     }
     __syncthreads();
     conv_bwd_layer<3, NI, 1, NI == 2 ? 5 : 3>(S.g4, S.t3, bw, a3 + b * kAct2, S.g3,
                                               g3 + b * kAct2, n);
     __syncthreads();
-    conv_bwd_layer<2, NI, 2, NI == 2 ? 5 : 3>(S.g3, S.t2, bw, a2 + b * kAct1, S.g2,
+    conv_bwd_layer<2, NI, 2, 3>(S.g3, S.t2, bw, a2 + b * kAct1, S.g2,
                                               g2 + b * kAct1, n);
     __syncthreads();
-    conv_bwd_layer<1, NI, 1, NI == 2 ? 5 : 5>(S.g2, S.t1, bw, a1 + b * kAct0, nullptr,
+    conv_bwd_layer<1, NI, 1, 5>(S.g2, S.t1, bw, a1 + b * kAct0, nullptr,
                                               g1 + b * kAct0, n);
   }
 }
