@@ -58,9 +58,9 @@ __constant__ unsigned char c_order[16] = {
     tet_order(6),  tet_order(7),  tet_order(8),  tet_order(9),  tet_order(10), tet_order(11),
     tet_order(12), tet_order(13), tet_order(14), tet_order(15)};
 
-// One warp extracts one brick; a block's warps share a list of its flagged
-// bricks. 7 blocks of 4 warps an SM (their shared memory) keep enough loads in
-// flight to hide the bricks' latency.
+// One warp extracts one brick, or one of `parts` shares of its cells; a block's
+// warps share a list of its flagged bricks. 7 blocks of 4 warps an SM (their
+// shared memory) keep enough loads in flight to hide the bricks' latency.
 constexpr int kMeshWarps = 4, kMeshThreads = 32 * kMeshWarps, kMeshBlocksPerSm = 7;
 constexpr int kMeshList = 512;   // flags a block looks through at a time
 constexpr int kEdge = 9;         // a brick's voxels and the next one along each axis
@@ -161,7 +161,7 @@ template <int STORAGE>
 __global__ void __launch_bounds__(kMeshThreads, kMeshBlocksPerSm)
     k_mesh(const uint32_t *__restrict__ vol, VolGeom g, float *__restrict__ tris,
            unsigned long long *__restrict__ ids, unsigned int max_tris,
-           unsigned int *__restrict__ count) {
+           unsigned int *__restrict__ count, int parts) {
   __shared__ MeshWarp s_warp[kMeshWarps];
   __shared__ int s_list[kMeshList];
   __shared__ int s_n, s_next;
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(kMeshThreads, kMeshBlocksPerSm)
       int e = 0;
       if (lane == 0) e = atomicAdd(&s_next, 1);
       e = __shfl_sync(0xffffffffu, e, 0);
-      if (e >= listed) break;
-      const int b = s_list[e];
+      if (e >= listed * parts) break;
+      const int b = s_list[e / parts], part = e % parts;
       const int bx = b / (nb * nb), by = (b / nb) % nb, bz = b % nb;
       // the brick's words, and whether one is observed at all
       const uint4 *src = reinterpret_cast<const uint4 *>(vol + ((size_t)b << 9)) + lane;
@@ -217,8 +217,9 @@ __global__ void __launch_bounds__(kMeshThreads, kMeshBlocksPerSm)
         }
       }
       __syncwarp();
-      const int items = active_cells<STORAGE>(s, lane) * 6;
-      if (items == 0) continue;
+      const int all = active_cells<STORAGE>(s, lane) * 6;
+      const int begin = all * part / parts, items = all * (part + 1) / parts;
+      if (items == begin) continue;
       // the brick's triangles, then their space in the output (one atomic)
       auto inside = [&](int it, int &x, int &y, int &z, uint32_t &tet) {
         const int c = s.cells[it / 6];
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kMeshThreads, kMeshBlocksPerSm)
         return ni == 0 || ni == 4 ? 0 : (ni == 2 ? 2 : 1);
       };
       int total = 0;
-      for (int it = lane; it < items; it += 32) {
+      for (int it = begin + lane; it < items; it += 32) {
         int x, y, z;
         uint32_t tet;
         total += triangles(inside(it, x, y, z, tet));
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kMeshThreads, kMeshBlocksPerSm)
       unsigned base = 0;
       if (lane == 0 && total > 0) base = atomicAdd(count, (unsigned)total);
       base = __shfl_sync(0xffffffffu, base, 0);
-      for (int i0 = 0; i0 < items; i0 += 32) {
+      for (int i0 = begin; i0 < items; i0 += 32) {
         const int it = i0 + lane;
         int x = 0, y = 0, z = 0, m = 0;
         uint32_t tet = 0;
@@ -330,14 +331,19 @@ extern "C" of_status_t of_mesh_extract(const of_volume_desc_t *d, const void *vo
   const VolGeom g = make_geom(*d);
   const int nbr = g.nb * g.nb * g.nb;
   const int blocks = nbr < kSmCount * kMeshBlocksPerSm ? nbr : kSmCount * kMeshBlocksPerSm;
+  // A small volume has fewer flagged bricks than the device has warps, and one
+  // warp's way through a brick's cells sets the time: four warps then share a
+  // brick's cells (each reads the brick). k_mesh at 104^3 44 -> 17 us, 176^3 47
+  // -> 24, 248^3 50 -> 29; at 304^3 65 -> 77, at 512^3 77 -> 105.
+  const int parts = nbr <= 8 * kMeshWarps * kMeshBlocksPerSm * kSmCount ? kMeshWarps : 1;
   if (d->storage == OF_TSDF_I16)
     k_mesh<OF_TSDF_I16><<<blocks, kMeshThreads, 0, s>>>((const uint32_t *)vol, g, d_tris,
                                                        (unsigned long long *)d_ids, max_triangles,
-                                                       d_count);
+                                                       d_count, parts);
   else
     k_mesh<OF_TSDF_F16><<<blocks, kMeshThreads, 0, s>>>((const uint32_t *)vol, g, d_tris,
                                                        (unsigned long long *)d_ids, max_triangles,
-                                                       d_count);
+                                                       d_count, parts);
   return of_launch_status();
 }
 
